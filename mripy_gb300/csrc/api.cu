@@ -82,6 +82,7 @@ struct gbn_plan {
     double tau = 0;
     Geom gs{}, gi{};
     int coil_group = 1, threads = 256, interp_threads = 256, max_sub = 256, interp_coil_group = 0;
+    int interp_max_sub = 1 << 30;  // interp work items where the spread's own size is longer
     int interp_staging = 0;  // 0: tensor copies where the grid allows, 1: thread loads
     int interp_variant = 0;  // 3-D, 8 coils: 0 library choice, 1 interp bins, 2 tensor cores
     int spread_variant = 0;  // 3-D, 8 coils: 0 library choice, 1 warp rows, 2 cubes, 3 tensor cores
@@ -321,7 +322,9 @@ int spread_cg(const gbn_plan *p) {
 // holds
 bool spread_interleaved(const gbn_plan *p) { return spread_reads_interleaved(p->gs, spread_cg(p), p->spread_variant); }
 
-int run_spread(gbn_plan *p, const void *c, gbn_layout L, const float *weight, float2 *grid, cudaStream_t s) {
+// real: the samples' imaginary parts are zero
+int run_spread(gbn_plan *p, const void *c, gbn_layout L, const float *weight, float2 *grid, cudaStream_t s,
+               bool real = false) {
     NvtxRange range("gbn spread");
     // tiles covered by several work items start from zero; when they are most of the grid
     // (dense trajectories), one memset of the whole grid is cheaper than per-tile blocks
@@ -346,6 +349,7 @@ int run_spread(gbn_plan *p, const void *c, gbn_layout L, const float *weight, fl
     a.n_dense = p->n_dense_sub;
     a.variant = p->spread_variant;
     a.status = p->kstatus;
+    a.real = real ? 1 : 0;
     const int cg = spread_cg(p);
     if (spread_smem_bytes(p->gs, cg) > (size_t)p->smem_optin)
         return fail(GBN_ERR_CAPACITY, "spread tile does not fit in shared memory");
@@ -367,6 +371,8 @@ int interp_cg(const gbn_plan *p) {
     int n_pow2 = 1;
     while (n_pow2 < n) n_pow2 *= 2;
     if (cg > n_pow2) cg = n_pow2;
+    // 3-D, up to 3 coils: a block per coil
+    if (cg <= 0 && p->dim == 3 && n <= 3 && interp3d_one_applies(p->gi)) cg = 1;
     if (cg <= 0) {
         int best = 1 << 30;
         for (int cand : {8, 4, 2, 1}) {
@@ -656,7 +662,7 @@ int set_points_impl(gbn_plan *p, int dtype, const void *x, const void *y, const 
     // items of at most that size stream each window once
     const int interp_max_sub = interp3d_planes_smem(p->gi, interp_cg(p), p->interp_threads) > 0
                                    ? std::min(p->max_sub, kPlaneSamples)
-                                   : p->max_sub;
+                                   : std::min(p->max_sub, p->interp_max_sub);
     SubsJob js{&p->gs, scount, &p->spread_tile_off, &p->nsub, &p->sub_off, 1, p->max_sub, dense_min,
                p->kstatus + 1, p->kstatus + 2};
     js.interleave = spread_interleaved(p) ? 1 : 0;
@@ -938,13 +944,28 @@ int plan_create_impl(const gbn_plan_desc *desc, gbn_plan **out) {
         ts[2] = 4 * (32 / cg_eff);
         reg_spread = true;
     }
+    // 3-D with 1 to 3 coils, unless the caller chose a tile or threads: the few-coil
+    // register kernel on its own tile.  Work items of 512 samples (measured: 768,000 samples
+    // 0.59, 0.52, 0.49, 0.47 ms at 128, 256, 512, 1024; 32,000 samples 47, 45, 50, 63 us)
+    bool few_spread = false;
+    if (p->dim == 3 && !tile_given && desc->threads <= 0 && (int)desc->n_coil <= kFewMaxCoils && p->ns <= 8) {
+        int tf[3];
+        few_tile(desc->n_coil, tf);
+        few_spread = true;
+        for (int d = 0; d < 3; ++d) few_spread = few_spread && p->nf[d] >= tf[d] + 2 * p->ns;
+        if (few_spread) {
+            for (int d = 0; d < 3; ++d) ts[d] = tf[d];
+            reg_spread = false;
+        }
+    }
     // the cube and tensor-core kernels keep a ring of batches full: long work items (the 3-D
     // tensor-core spread and interp share the work items; measured on the 3-D radial
     // workload: interp 3.75 ms at 4096 samples against 3.93 at 2048, spread even)
     const bool cube = cg_eff == 8 && ((p->dim == 3 && p->spread_variant == 2) || p->spread_variant == 3);
     const bool mma3 = cube && p->dim == 3 && p->spread_variant == 3;
     p->max_sub = desc->max_subproblem > 0 ? desc->max_subproblem
-                                          : (mma3 ? 4096 : (cube ? 2048 : (reg_spread && p->dim == 2 ? 128 : 256)));
+                                          : (mma3 ? 4096 : (cube ? 2048 : (few_spread ? 512 : (reg_spread && p->dim == 2 ? 128 : 256))));
+    if (few_spread && desc->max_subproblem <= 0) p->interp_max_sub = 256;
     make_geom(p, ts, p->gs);
     make_geom(p, ti, p->gi);
 
@@ -1500,7 +1521,7 @@ int gbn_dcf_pipe_menon(gbn_plan *p, int32_t n_iter, float *dcf, gbn_stream_t str
     const gbn_layout cl = {0, 1, 1};
     GBN_CUDA(launch_dcf_fill(w, p->M, s));
     for (int it = 0; it < n_iter; ++it) {
-        GBN_TRY(run_spread(p, w, cl, nullptr, p->grid, s));
+        GBN_TRY(run_spread(p, w, cl, nullptr, p->grid, s, true));  // real weights
         GBN_TRY(run_interp(p, p->grid, cw, cl, nullptr, s));
         GBN_CUDA(launch_dcf_update(w, cw, p->M, s));
     }

@@ -137,6 +137,7 @@ struct SpreadArgs {
     int any_dense;            // some subproblems carry kDenseFlag (compensated accumulation)
     const uint32_t *dense_subs;  // the indices of those subproblems (n_dense of them)
     int64_t n_dense;
+    int real = 0;             // the samples' imaginary parts are zero (density compensation)
     int variant;              // 3-D, 8 coils: 0 library choice, 1 warp rows, 2 cubes (gbn_plan_desc)
     uint32_t *status;         // the plan's status word (bounded waits of the cube kernel)
 };
@@ -185,6 +186,10 @@ cudaError_t launch_spread(const SpreadArgs &a, int64_t n_sub, int coil_group, in
 bool spread_reads_interleaved(const Geom &g, int coil_group, int variant);
 // the 3-D 8-coil spread kernel launch_spread runs: 3 tensor cores, 2 cubes, 1 warp rows, 0 other
 int spread_path_kind(const Geom &g, int coil_group, int variant, int threads);
+// the few-coil 3-D spread (spread3d_few.cuh) takes this spread geometry: 1 to 3 coils, its tile
+constexpr int kFewMaxCoils = 3;
+bool few_applies(const Geom &g);
+void few_tile(int n_coil, int tile[3]);
 // kernels launch_spread runs for these arguments (the 3-D register path adds a Kahan instance)
 int spread_kernel_count(const SpreadArgs &a, int64_t n_sub, int coil_group, int threads);
 cudaError_t launch_interp(const InterpArgs &a, int64_t n_sub, int coil_group, int threads,
@@ -195,6 +200,8 @@ size_t spread_smem_bytes(const Geom &g, int coil_group);
 size_t interp_smem_bytes(const Geom &g, int coil_group, int threads);
 // shared memory of the plane-streaming 3-D interp, 0 where it does not apply
 size_t interp3d_planes_smem(const Geom &g, int coil_group, int threads);
+// the one-coil 3-D interp (interp3d_one.cuh) takes this geometry
+bool interp3d_one_applies(const Geom &g);
 constexpr int kPlaneSamples = 64;  // samples per chunk of the plane-streaming 3-D interp
 // plane box (y rows, z cells per coil) of the plane-streaming 3-D interp: the tensor copy's
 // box over a grid tensor map (z, y, x, instance); false where the kernel does not apply

@@ -44,6 +44,14 @@ __device__ __forceinline__ int wrap_fast(int v, int n) {
 // 2^-21 (a/b) of the true quotient, far less than the 0.5/b to the nearest integer
 __device__ __forceinline__ int div_small(int a, float rb) { return (int)(((float)a + 0.5f) * rb); }
 
+// 2^x (PTX ex2.approx, flushing subnormal results to zero: the Gaussian's smallest weight
+// inside the stencil is ~eps, far above the subnormal range)
+__device__ __forceinline__ float ex2_approx(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // --------------------------------------------------------------------------------- interp
 template <int WT, int CG>
 __global__ void __launch_bounds__(512) k_interp2d(InterpArgs a) {

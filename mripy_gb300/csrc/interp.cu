@@ -3,7 +3,8 @@
 // 2-D with at most 16 taps per dimension: k_interp2d_tma (persistent, windows staged by
 // tensor copies; the caller supplies the tensor map) or k_interp2d (one block per
 // subproblem, windows gathered by the threads).  3-D with at most 16 taps:
-// k_interp3d_planes (4 or 8 coils per block, window streamed by x planes) or k_interp3d.
+// k_interp3d_one (one coil per block: plans of 1 to 3 coils), k_interp3d_planes (4 or 8 coils
+// per block, window streamed by x planes) or k_interp3d.
 // Otherwise (1-D, wide stencils): k_interp (one thread per sample).
 #include <algorithm>
 #include <cstring>
@@ -13,6 +14,7 @@
 #include "grid3d_kernels.cuh"
 #include "interp2d_tma.cuh"
 #include "interp3d_mma.cuh"
+#include "interp3d_one.cuh"
 
 namespace gbn {
 
@@ -22,11 +24,18 @@ size_t interp3d_planes_smem(const Geom &g, int coil_group, int threads) {
     return interp3d_planes_smem_bytes(g, coil_group, threads > 256 ? 256 : threads);
 }
 
+// one coil per block in 3-D: the paired-cell kernel, while two blocks' windows fit an SM
+bool interp3d_one_applies(const Geom &g) {
+    const size_t b = interp3d_one_smem_bytes(g);
+    return b > 0 && b <= 112 * 1024;
+}
+
 // shared memory of the kernel launch_interp runs for this geometry, coil group and thread
 // count (the 3-D kernel depends on all three)
 size_t interp_smem_bytes(const Geom &g, int coil_group, int threads) {
     if (use_2d_path(g)) return interp2d_smem_bytes(g, coil_group);
     if (const size_t ps = interp3d_planes_smem_bytes(g, coil_group, threads > 256 ? 256 : threads)) return ps;
+    if (coil_group == 1 && interp3d_one_applies(g)) return interp3d_one_smem_bytes(g);
     size_t cells = 1;
     for (int d = 0; d < g.dim; ++d) cells *= (size_t)(g.tile[d] + g.W - 1);
     return cells * (size_t)coil_group * sizeof(float2);
@@ -89,6 +98,18 @@ cudaError_t launch_interp(const InterpArgs &a, int64_t n_sub, int coil_group, in
         const int th = threads > 256 ? 256 : threads;
         if (interp3d_planes_smem_bytes(a.g, coil_group, th))  // 4 or 8 coils: stream plane by plane
             return launch_interp3d_planes(a, n_sub, coil_group, th, nullptr, nullptr, s);
+        if (coil_group == 1 && interp3d_one_applies(a.g)) {
+            const int vec = (uintptr_t)a.grid % 16 == 0 && a.g.nf[2] % 2 == 0 && a.g.G % 2 == 0;
+            GBN_DISPATCH_W(a.g.W, {
+                auto kern = k_interp3d_one<WT>;
+                err = set_smem(kern, smem);
+                if (err == cudaSuccess) {
+                    kern<<<grid, th, smem, s>>>(a, vec);
+                    err = cudaGetLastError();
+                }
+            });
+            return err;
+        }
         const size_t wsmem = interp3d_smem_bytes(a.g, coil_group);  // the whole staged window
         GBN_DISPATCH_W(a.g.W, GBN_DISPATCH_CG(coil_group, {
             auto kern = k_interp3d<WT, CG>;

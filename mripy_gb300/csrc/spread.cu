@@ -11,6 +11,7 @@
 #include "grid2d_kernels.cuh"
 #include "grid3d_kernels.cuh"
 #include "spread3d_cube.cuh"
+#include "spread3d_few.cuh"
 #include "spread3d_mma.cuh"
 
 #include <algorithm>
@@ -64,6 +65,18 @@ static bool mma_path(const Geom &g, int coil_group, int variant) {
     if (g.dim == 3)
         return grid3d_applies(g) && g.tile[0] == kMmaTX && g.tile[1] == kMmaTY && g.tile[2] == kMmaTZ;
     return use_2d_path(g) && g.tile[0] == kMmaTY && g.tile[1] == kMmaTZ;
+}
+
+// the few-coil 3-D kernel applies: 1 to 3 coils, its tile, a grid of at least tile + stencil
+// cells per axis.  Four coils and more keep the kernels that sum dense tiles with compensation.
+bool few_applies(const Geom &g) {
+    return g.dim == 3 && g.n_coil >= 1 && g.n_coil <= kFewMaxCoils && grid3d_applies(g) && g.tile[0] == kFewTile &&
+           g.tile[1] == kFewTile && g.tile[2] == few_tz(g.n_coil);
+}
+
+void few_tile(int n_coil, int tile[3]) {
+    tile[0] = tile[1] = kFewTile;
+    tile[2] = few_tz(n_coil);
 }
 
 // the cube and tensor-core kernels read interleaved work items
@@ -154,6 +167,18 @@ cudaError_t launch_spread(const SpreadArgs &a, int64_t n_sub, int coil_group, in
     // tensor-core kernel (8 coils per block; 3-D: then compensated sums for dense units)
     if (mma_path(a.g, coil_group, a.variant)) {
         GBN_DISPATCH_W(a.g.W, { err = launch_mma<WT>(a, n_sub, s); });
+        return err;
+    }
+    // few-coil 3-D kernel
+    if (few_applies(a.g)) {
+        const int nc = a.g.n_coil;
+        GBN_DISPATCH_W(a.g.W, {
+            auto kern = nc == 1   ? (a.real ? k_spread3d_few<WT, 1, true> : k_spread3d_few<WT, 1, false>)
+                        : nc == 2 ? k_spread3d_few<WT, 2, false>
+                                  : k_spread3d_few<WT, 3, false>;
+            kern<<<(unsigned)n_sub, kFewWarps * 32, few_smem_bytes(nc), s>>>(a);
+            err = cudaGetLastError();
+        });
         return err;
     }
     // register-tile kernel: 4 or 8 coils per block and the tile it is built for

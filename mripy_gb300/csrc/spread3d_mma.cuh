@@ -116,13 +116,6 @@ template <> struct MmaTile<2> {
 };
 template <int D> constexpr int mma_n() { return MmaTile<D>::NX * 16; }
 
-// 2^x (PTX ex2.approx, flushing subnormal results to zero: the Gaussian's smallest weight
-// inside the stencil is ~eps, far above the subnormal range)
-__device__ __forceinline__ float ex2_approx(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 
 // Two products x = a * b (one packed FP32x2 multiply) split as x = hi + lo: hi rounded to
 // the TF32 grid (11 significant bits; ties away from zero, by integer arithmetic on the bit

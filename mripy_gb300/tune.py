@@ -47,6 +47,8 @@ def _spread_candidates(dim, n_coil):
             out.append(((4, 8, 16), 256, 8, 3))
             for tile in ((8, 8, 8), (4, 8, 16), (8, 8, 16), (16, 8, 8)):
                 out.append((tile, 256, 8, 2))
+        if n_coil < 4:  # the few-coil register kernel's tile
+            out.append(((8, 8, 16 if n_coil == 1 else 8), 256, 8, 0))
         out += [((8, 8, 32), 256, 8, 0)]
     else:
         out = [((t,), 256, 8, 0) for t in (1024, 512, 2048)]
