@@ -112,6 +112,12 @@ struct gbn_plan {
     bool fft_x_ok = false;
     void *fft_work = nullptr;
 
+    // the composite calls' transforms with pad and crop fused in (fft_variant 0, every grid
+    // length among the supported ones)
+    bool own_fft = false;
+    BandFft own{};
+    float2 *own_tw = nullptr;
+
     // tensor map of the last grid the TMA interp read (re-encoded when the grid changes)
     CUtensorMap tmap{};
     const void *tmap_grid = nullptr;
@@ -301,14 +307,47 @@ int fft_band_exec(gbn_plan *p, float2 *grid, int direction, int band, cudaStream
     return planes();
 }
 
+int dir_type1(const gbn_plan *p) { return p->desc.iflag < 0 ? GBN_FFT_FORWARD : GBN_FFT_INVERSE; }
+int dir_type2(const gbn_plan *p) { return p->desc.iflag < 0 ? GBN_FFT_INVERSE : GBN_FFT_FORWARD; }
+
+// image (SENSE image and maps) -> deapodised, padded, transformed grid
+int image_to_grid(gbn_plan *p, const void *img, gbn_layout L, const void *sens, gbn_layout SL, cudaStream_t s) {
+    const DeapodArgs a = deapod_args(p, false);
+    const float2 *x = (const float2 *)img, *m = (const float2 *)sens;
+    if (p->own_fft) {
+        GBN_CUDA(launch_band_fft_in(p->own, a, dir_type2(p) < 0 ? 0 : 1, x, L, m, SL, p->grid, s));
+        return GBN_OK;
+    }
+    if (m)
+        GBN_CUDA(launch_pad_sense(a, x, L, m, SL, p->grid, s));
+    else
+        GBN_CUDA(launch_pad(a, x, L, p->grid, s));
+    return fft_band_exec(p, p->grid, dir_type2(p), GBN_BAND_INPUT, s);
+}
+
+// spread grid -> transformed, cropped, deapodised image (summed over the coils with the maps'
+// conjugates)
+int grid_to_image(gbn_plan *p, void *img, gbn_layout L, const void *sens, gbn_layout SL, cudaStream_t s) {
+    const DeapodArgs a = deapod_args(p, true);
+    float2 *x = (float2 *)img;
+    const float2 *m = (const float2 *)sens;
+    if (p->own_fft) {
+        GBN_CUDA(launch_band_fft_out(p->own, a, dir_type1(p) < 0 ? 0 : 1, p->grid, x, L, m, SL, s));
+        return GBN_OK;
+    }
+    GBN_TRY(fft_band_exec(p, p->grid, dir_type1(p), GBN_BAND_OUTPUT, s));
+    if (m)
+        GBN_CUDA(launch_crop_sense(a, p->grid, m, SL, x, L, s));
+    else
+        GBN_CUDA(launch_crop(a, p->grid, x, L, s));
+    return GBN_OK;
+}
+
 // shared memory a block may take when choosing coils per block: in 3-D two blocks per SM
 // (latency hiding) beat more coils per block
 size_t smem_budget(const gbn_plan *p) {
     return p->dim == 3 ? std::min<size_t>((size_t)p->smem_optin, 116 * 1024) : (size_t)p->smem_optin;
 }
-
-int dir_type1(const gbn_plan *p) { return p->desc.iflag < 0 ? GBN_FFT_FORWARD : GBN_FFT_INVERSE; }
-int dir_type2(const gbn_plan *p) { return p->desc.iflag < 0 ? GBN_FFT_INVERSE : GBN_FFT_FORWARD; }
 
 // coils per spread block: the plan's group, capped at the coil count and by shared memory
 int spread_cg(const gbn_plan *p) {
@@ -816,6 +855,31 @@ void drop_fft_band(gbn_plan *p) {
     p->fft_band = false;
 }
 
+// Whether the composite calls run the fused transforms, and their twiddle tables.
+int make_own_fft(gbn_plan *p) {
+    if (p->fft_variant != 0 || p->dim < 2 || p->G > 0x7FFFFFFF) return GBN_OK;
+    for (int d = 0; d < p->dim; ++d) {
+        p->own.e[d] = fft_entry(p->nf[d]);
+        if (!p->own.e[d]) return GBN_OK;
+    }
+    // blocks of the widest launch
+    if ((double)p->n_inst * p->nf[0] * std::max(p->nf[1], 16) / 16 * std::max(p->nf[2], 16) / 8 > 2e9) return GBN_OK;
+    size_t cells = 0;
+    for (int d = 0; d < p->dim; ++d) cells += (size_t)p->nf[d];
+    GBN_CUDA(cudaMalloc((void **)&p->own_tw, sizeof(float2) * cells));
+    p->device_bytes += sizeof(float2) * cells;
+    float2 *tw = p->own_tw;
+    for (int d = 0; d < p->dim; ++d) {
+        GBN_CUDA(fft_prepare(*p->own.e[d]));
+        p->own.tw[d] = tw;
+        GBN_CUDA(launch_fft_twiddles(p->nf[d], tw, 0));
+        tw += p->nf[d];
+    }
+    GBN_CUDA(cudaStreamSynchronize(0));
+    p->own_fft = true;
+    return GBN_OK;
+}
+
 int plan_create_impl(const gbn_plan_desc *desc, gbn_plan **out) {
     if (!desc || !out) return fail(GBN_ERR_ARG, "null argument");
     *out = nullptr;
@@ -1029,6 +1093,8 @@ int plan_create_impl(const gbn_plan_desc *desc, gbn_plan **out) {
             drop_fft_band(p);  // the library's choice: the full transform instead
         }
     }
+    const int st_own = make_own_fft(p);
+    if (st_own != GBN_OK) return bail(st_own);
     *out = p;
     return GBN_OK;
 }
@@ -1081,6 +1147,7 @@ int gbn_plan_destroy(gbn_plan *p) {
     for (int i = 0; i < p->fft_n_planes; ++i) cufftDestroy(p->fft_planes[i]);
     if (p->fft_x_ok) cufftDestroy(p->fft_x);
     if (p->fft_work) cudaFree(p->fft_work);
+    if (p->own_tw) cudaFree(p->own_tw);
     if (p->grid) cudaFree(p->grid);
     if (p->kstatus) cudaFree(p->kstatus);
     for (int d = 0; d < 3; ++d)
@@ -1223,17 +1290,14 @@ int gbn_type1(gbn_plan *p, const void *c, gbn_layout cl, const float *weight, vo
     if ((!c && p->M > 0) || !img) return fail(GBN_ERR_ARG, "null buffer");
     cudaStream_t s = (cudaStream_t)stream;
     GBN_TRY(run_spread(p, c, cl, weight, p->grid, s));
-    GBN_TRY(fft_band_exec(p, p->grid, dir_type1(p), GBN_BAND_OUTPUT, s));
-    GBN_CUDA(launch_crop(deapod_args(p, true), p->grid, (float2 *)img, il, s));
-    return GBN_OK;
+    return grid_to_image(p, img, il, nullptr, gbn_layout{}, s);
 }
 
 int gbn_type2(gbn_plan *p, const void *img, gbn_layout il, void *c, gbn_layout cl, gbn_stream_t stream) {
     GBN_TRY(check_plan(p, true));
     if ((!c && p->M > 0) || !img) return fail(GBN_ERR_ARG, "null buffer");
     cudaStream_t s = (cudaStream_t)stream;
-    GBN_CUDA(launch_pad(deapod_args(p, false), (const float2 *)img, il, p->grid, s));
-    GBN_TRY(fft_band_exec(p, p->grid, dir_type2(p), GBN_BAND_INPUT, s));
+    GBN_TRY(image_to_grid(p, img, il, nullptr, gbn_layout{}, s));
     GBN_TRY(run_interp(p, p->grid, c, cl, nullptr, s));
     return GBN_OK;
 }
@@ -1244,13 +1308,10 @@ int gbn_type21(gbn_plan *p, const void *img, gbn_layout il, void *out, gbn_layou
     if (!img || !out) return fail(GBN_ERR_ARG, "null buffer");
     cudaStream_t s = (cudaStream_t)stream;
     const gbn_layout sl = {0, 1, p->desc.n_coil};
-    GBN_CUDA(launch_pad(deapod_args(p, false), (const float2 *)img, il, p->grid, s));
-    GBN_TRY(fft_band_exec(p, p->grid, dir_type2(p), GBN_BAND_INPUT, s));
+    GBN_TRY(image_to_grid(p, img, il, nullptr, gbn_layout{}, s));
     GBN_TRY(run_interp(p, p->grid, p->scratch.p, sl, dcf, s));
     GBN_TRY(run_spread(p, p->scratch.p, sl, nullptr, p->grid, s));
-    GBN_TRY(fft_band_exec(p, p->grid, dir_type1(p), GBN_BAND_OUTPUT, s));
-    GBN_CUDA(launch_crop(deapod_args(p, true), p->grid, (float2 *)out, ol, s));
-    return GBN_OK;
+    return grid_to_image(p, out, ol, nullptr, gbn_layout{}, s);
 }
 
 int gbn_sense_forward(gbn_plan *p, const void *x, gbn_layout xl, const void *sens, gbn_layout sl, void *kdata,
@@ -1258,8 +1319,7 @@ int gbn_sense_forward(gbn_plan *p, const void *x, gbn_layout xl, const void *sen
     GBN_TRY(check_plan(p, true));
     if (!x || !sens || (!kdata && p->M > 0)) return fail(GBN_ERR_ARG, "null buffer");
     cudaStream_t s = (cudaStream_t)stream;
-    GBN_CUDA(launch_pad_sense(deapod_args(p, false), (const float2 *)x, xl, (const float2 *)sens, sl, p->grid, s));
-    GBN_TRY(fft_band_exec(p, p->grid, dir_type2(p), GBN_BAND_INPUT, s));
+    GBN_TRY(image_to_grid(p, x, xl, sens, sl, s));
     GBN_TRY(run_interp(p, p->grid, kdata, kl, nullptr, s));
     return GBN_OK;
 }
@@ -1270,9 +1330,7 @@ int gbn_sense_adjoint(gbn_plan *p, const void *kdata, gbn_layout kl, const float
     if (!x || !sens || (!kdata && p->M > 0)) return fail(GBN_ERR_ARG, "null buffer");
     cudaStream_t s = (cudaStream_t)stream;
     GBN_TRY(run_spread(p, kdata, kl, dcf, p->grid, s));
-    GBN_TRY(fft_band_exec(p, p->grid, dir_type1(p), GBN_BAND_OUTPUT, s));
-    GBN_CUDA(launch_crop_sense(deapod_args(p, true), p->grid, (const float2 *)sens, sl, (float2 *)x, xl, s));
-    return GBN_OK;
+    return grid_to_image(p, x, xl, sens, sl, s);
 }
 
 int gbn_sense_normal(gbn_plan *p, const void *x, gbn_layout xl, const void *sens, gbn_layout sl,
@@ -1281,13 +1339,10 @@ int gbn_sense_normal(gbn_plan *p, const void *x, gbn_layout xl, const void *sens
     if (!x || !sens || !x_out) return fail(GBN_ERR_ARG, "null buffer");
     cudaStream_t s = (cudaStream_t)stream;
     const gbn_layout scl = {0, 1, p->desc.n_coil};
-    GBN_CUDA(launch_pad_sense(deapod_args(p, false), (const float2 *)x, xl, (const float2 *)sens, sl, p->grid, s));
-    GBN_TRY(fft_band_exec(p, p->grid, dir_type2(p), GBN_BAND_INPUT, s));
+    GBN_TRY(image_to_grid(p, x, xl, sens, sl, s));
     GBN_TRY(run_interp(p, p->grid, p->scratch.p, scl, dcf, s));
     GBN_TRY(run_spread(p, p->scratch.p, scl, nullptr, p->grid, s));
-    GBN_TRY(fft_band_exec(p, p->grid, dir_type1(p), GBN_BAND_OUTPUT, s));
-    GBN_CUDA(launch_crop_sense(deapod_args(p, true), p->grid, (const float2 *)sens, sl, (float2 *)x_out, ol, s));
-    return GBN_OK;
+    return grid_to_image(p, x_out, ol, sens, sl, s);
 }
 
 int gbn_interp_grad_coords(gbn_plan *p, const void *grid, const void *grad_c, gbn_layout cl, float *grad_xyz,

@@ -235,6 +235,8 @@ struct DeapodArgs {
 };
 cudaError_t launch_build_tables(int dim, const int m[3], const int nf[3], double tau, float *tab0,
                                 float *tab1, float *tab2, cudaStream_t s);
+// coils a block should read or write together when the image is in host memory (1: no such bound)
+int host_min_cc(const void *img, bool coil_fast, int n_coil, cudaStream_t s);
 cudaError_t launch_pad(const DeapodArgs &a, const float2 *img, gbn_layout L, float2 *grid,
                        cudaStream_t s);
 cudaError_t launch_crop(const DeapodArgs &a, const float2 *grid, float2 *img, gbn_layout L,
@@ -243,6 +245,54 @@ cudaError_t launch_pad_sense(const DeapodArgs &a, const float2 *x, gbn_layout XL
                              gbn_layout SL, float2 *grid, cudaStream_t s);
 cudaError_t launch_crop_sense(const DeapodArgs &a, const float2 *grid, const float2 *sens,
                               gbn_layout SL, float2 *x, gbn_layout XL, cudaStream_t s);
+
+// band_fft.cuh: transforms with pad and crop fused in
+constexpr int kFftLines = 16;  // lines per block
+struct FftCols {               // one strided axis, in place
+    int64_t G, stride;         // cells per instance; cells between neighbours along the axis
+    int cols, chunks;          // inner cells, blocks of kFftLines of them
+    int n_sub, sub_lo;         // sub-volumes per instance: 0 .. sub_lo - 1, then those after
+    int64_t sub_skip, sub_stride;  // sub_skip further ones
+    int lo, hi;                // the axis' band: cells [0, lo) and [N - hi, N)
+    const float2 *tw;          // exp(-2 pi i k / N)
+    int inv;
+};
+enum { kFftRowsIn, kFftRowsOut, kFftRowsSense };
+struct FftRows {               // the contiguous axis, between image and grid
+    int64_t G;
+    int n_rows, rows_per_grp;  // rows = (group, outer pixels)
+    int n_coil, m0, m1, nf0, nf1;     // outer axes (m1 = 1 in 2-D)
+    int m, nf, lo, hi;         // the axis: image size, grid size, band
+    int rpb, cpc, n_chunk;     // image rows per block, coils per chunk, chunks
+    int lfast;                 // image side: coils of a pixel adjacent
+    const float *tab0, *tab1, *tab;   // deapodisation tables (tab1 null in 2-D)
+    const float *grp_scale;    // rows out
+    const float2 *tw;
+    int inv;
+    const float2 *img;         // rows in: image, or SENSE image with sens
+    float2 *out;               // rows out
+    gbn_layout IL;
+    const float2 *sens;
+    gbn_layout SL;
+};
+struct FftEntry {              // the kernels of one length
+    int n;
+    cudaError_t (*prepare)();  // raises their shared-memory limits
+    cudaError_t (*cols)(float2 *grid, const FftCols &a, int64_t blocks, bool out, cudaStream_t s);
+    cudaError_t (*rows)(float2 *grid, const FftRows &a, int64_t blocks, int kind, cudaStream_t s);
+};
+const FftEntry *fft_entry(int n);  // null where the length has no kernels
+cudaError_t fft_prepare(const FftEntry &e);  // prepare(), once per device
+cudaError_t launch_fft_twiddles(int n, float2 *tw, cudaStream_t s);
+// image (or SENSE image times maps) -> transformed grid, and back; tw: per axis, e: per axis
+struct BandFft {
+    const FftEntry *e[3];
+    const float2 *tw[3];
+};
+cudaError_t launch_band_fft_in(const BandFft &b, const DeapodArgs &a, int inv, const float2 *img, gbn_layout L,
+                               const float2 *sens, gbn_layout SL, float2 *grid, cudaStream_t s);
+cudaError_t launch_band_fft_out(const BandFft &b, const DeapodArgs &a, int inv, float2 *grid, float2 *img, gbn_layout L,
+                                const float2 *sens, gbn_layout SL, cudaStream_t s);
 
 // solver.cu: vector kernels of the CG and IST/FISTA solvers
 // Scalars of one solve, kept in device memory so no iteration waits on the host.

@@ -25,6 +25,26 @@
 
 namespace gbn {
 
+// Coils per chunk for an image in host memory (pinned, read or written by the kernel over
+// the host link): with coils fastest, 8 coils keep each pixel's 64-byte run in one block;
+// 2-coil chunks (16-byte pieces) made the c2 host-buffer step 25 % slower.
+// The query is skipped while the stream is being captured into a graph (host-buffer calls
+// are never captured).
+int host_min_cc(const void *img, bool coil_fast, int n_coil, cudaStream_t s) {
+    if (!coil_fast) return 1;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return 1;
+    }
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, img) != cudaSuccess) {
+        cudaGetLastError();
+        return 1;
+    }
+    return at.type == cudaMemoryTypeHost ? std::min(8, n_coil) : 1;
+}
+
 namespace {
 
 constexpr int kStageElems = 4096;  // staged complex values per band block (32 KB)
@@ -378,26 +398,6 @@ bool empty(const DeapodArgs &a) {
     for (int d = 0; d < a.g.dim; ++d)
         if (a.m[d] == 0) return true;
     return false;
-}
-
-// Coils per chunk for an image in host memory (pinned, read or written by the kernel over
-// the host link): with coils fastest, 8 coils keep each pixel's 64-byte run in one block;
-// 2-coil chunks (16-byte pieces) made the c2 host-buffer step 25 % slower.
-// The query is skipped while the stream is being captured into a graph (host-buffer calls
-// are never captured).
-int host_min_cc(const void *img, bool coil_fast, int n_coil, cudaStream_t s) {
-    if (!coil_fast) return 1;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
-        cudaGetLastError();
-        return 1;
-    }
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, img) != cudaSuccess) {
-        cudaGetLastError();
-        return 1;
-    }
-    return at.type == cudaMemoryTypeHost ? std::min(8, n_coil) : 1;
 }
 
 cudaError_t check_blocks(int64_t n) {
