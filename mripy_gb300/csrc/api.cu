@@ -127,9 +127,9 @@ struct gbn_plan {
     bool points_set = false;
     int64_t M = 0;
     std::vector<int64_t> traj_off;
-    DevBuf traj_off_d, grp_scale, pts, home_key, home_keys_sorted, touch_count, touch_off, home_count,
-        iota, home_idx, home_pts, dup_keys, dup_vals, dup_keys_sorted, dup_idx, dup_pts, spread_count,
-        spread_tile_off, home_tile_off, nsub, sub_off, nsub_i, sub_off_i, spread_subs, interp_subs, cub_tmp, scratch,
+    DevBuf traj_off_d, grp_scale, pts, home_key, home_keys_sorted, touch_count, touch_off, counts,
+        iota, home_idx, home_pts, dup_keys, dup_vals, dup_keys_sorted, dup_idx, dup_pts, spread_tile_off,
+        home_tile_off, sub_off, sub_off_i, spread_subs, interp_subs, cub_tmp, scratch,
         stage_in, stage_out, stage_w, split_tiles, dense_subs;
     int64_t n_dup = 0, n_spread_sub = 0, n_interp_sub = 0;
     int spread_kernels = 0;   // kernels the last spread launched (split-tile zeroing included)
@@ -566,61 +566,6 @@ int key_bits(uint64_t max_key) {
     return b;
 }
 
-// count -> tile offsets (exclusive), subproblem table
-// Work items of one bin geometry, in two phases so that the spread's and the interp's
-// totals (and the dense / split counts) come back to the host in one synchronisation.
-struct SubsJob {
-    const Geom *g;
-    uint32_t *count;      // samples per tile
-    DevBuf *tile_off;     // their exclusive scan
-    DevBuf *nsub;         // work items per tile
-    DevBuf *sub_off;      // their exclusive scan
-    int every_tile, max_sub;
-    uint32_t dense_min;
-    uint32_t *n_dense, *n_split;  // device counters (may be null)
-    int interleave = 0;           // split tiles' items take every s-th entry
-    int64_t T = 0;
-};
-
-// scans and per-tile item counts; the last tile's offset and count are copied into last[2]
-int subs_count(gbn_plan *p, SubsJob &j, uint32_t last[2], cudaStream_t s) {
-    j.T = (int64_t)j.g->ntiles * j.g->n_traj;
-    const int64_t T = j.T;
-    GBN_TRY(ensure(p, *j.tile_off, sizeof(uint32_t) * T));
-    GBN_TRY(ensure(p, *j.nsub, sizeof(uint32_t) * T));
-    GBN_TRY(ensure(p, *j.sub_off, sizeof(uint32_t) * (T + 1)));
-    uint32_t *toff = j.tile_off->as<uint32_t>(), *ns_ = j.nsub->as<uint32_t>(), *soff = j.sub_off->as<uint32_t>();
-    GBN_TRY(cub_call(p, [&](void *tmp, size_t &bytes) {
-        return cub::DeviceScan::ExclusiveSum(tmp, bytes, j.count, toff, (int)T, s);
-    }));
-    GBN_CUDA(launch_count_subs(j.count, T, j.max_sub, j.every_tile, j.dense_min, ns_, j.n_dense, j.n_split, s));
-    GBN_TRY(cub_call(p, [&](void *tmp, size_t &bytes) {
-        return cub::DeviceScan::ExclusiveSum(tmp, bytes, ns_, soff, (int)T, s);
-    }));
-    GBN_CUDA(cudaMemcpyAsync(&last[0], soff + (T - 1), sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    GBN_CUDA(cudaMemcpyAsync(&last[1], ns_ + (T - 1), sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    return GBN_OK;
-}
-
-// after the synchronisation: allocate and fill the work items
-int subs_build(gbn_plan *p, const SubsJob &j, const uint32_t last[2], DevBuf &subs, uint32_t *split_list,
-               uint32_t *split_cursor, uint32_t *dense_list, uint32_t *dense_cursor, int64_t *n_sub_out,
-               cudaStream_t s) {
-    const int64_t n_sub = (int64_t)last[0] + last[1];
-    if (n_sub > 0x7FFFFFFF) return fail(GBN_ERR_CAPACITY, "too many subproblems");
-    GBN_TRY(ensure(p, subs, sizeof(int4) * (size_t)std::max<int64_t>(n_sub, 1)));
-    GBN_CUDA(launch_build_subs(j.count, j.tile_off->as<uint32_t>(), j.sub_off->as<uint32_t>(), j.T, j.max_sub,
-                               j.every_tile, j.dense_min, j.interleave, split_list, split_cursor, dense_list,
-                               dense_cursor, subs.as<int4>(), s));
-    *n_sub_out = n_sub;
-    return GBN_OK;
-}
-
-__global__ void k_iota(uint32_t *v, int64_t n) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < n) v[i] = (uint32_t)i;
-}
-
 int set_points_impl(gbn_plan *p, int dtype, const void *x, const void *y, const void *z, const int64_t *off,
                     cudaStream_t s) {
     NvtxRange range("gbn set_points");
@@ -642,6 +587,8 @@ int set_points_impl(gbn_plan *p, int dtype, const void *x, const void *y, const 
 
     const size_t Mb = (size_t)std::max<int64_t>(M, 1);
     const int64_t Ti = (int64_t)p->gi.ntiles * nt, Ts = (int64_t)p->gs.ntiles * nt;
+    // one buffer, zeroed by one memset: totals and status, counts per interp bin and spread tile
+    const size_t count_bytes = sizeof(TileTotals) + sizeof(uint32_t) * (size_t)(Ti + Ts);
     GBN_TRY(ensure(p, p->traj_off_d, sizeof(int64_t) * (nt + 1)));
     GBN_TRY(ensure(p, p->grp_scale, sizeof(float) * nt));
     GBN_TRY(ensure(p, p->pts, sizeof(float4) * Mb));
@@ -649,27 +596,75 @@ int set_points_impl(gbn_plan *p, int dtype, const void *x, const void *y, const 
     GBN_TRY(ensure(p, p->home_keys_sorted, sizeof(uint32_t) * Mb));
     GBN_TRY(ensure(p, p->touch_count, sizeof(uint32_t) * Mb));
     GBN_TRY(ensure(p, p->touch_off, sizeof(uint64_t) * Mb));
-    GBN_TRY(ensure(p, p->home_count, sizeof(uint32_t) * (Ti + 1)));  // + status word
+    GBN_TRY(ensure(p, p->counts, count_bytes));
     GBN_TRY(ensure(p, p->iota, sizeof(uint32_t) * Mb));
     GBN_TRY(ensure(p, p->home_idx, sizeof(uint32_t) * Mb));
     GBN_TRY(ensure(p, p->home_pts, sizeof(float4) * Mb));
-    GBN_TRY(ensure(p, p->spread_count, sizeof(uint32_t) * Ts));
     GBN_TRY(ensure(p, p->scratch, sizeof(float2) * Mb * (size_t)p->desc.n_coil));
+    GBN_TRY(ensure(p, p->split_tiles, sizeof(uint32_t) * (size_t)std::max<int64_t>(Ts, 1)));
+    GBN_TRY(ensure(p, p->spread_tile_off, sizeof(uint32_t) * (size_t)Ts));
+    GBN_TRY(ensure(p, p->sub_off, sizeof(uint32_t) * (size_t)Ts));
+    GBN_TRY(ensure(p, p->home_tile_off, sizeof(uint32_t) * (size_t)Ti));
+    GBN_TRY(ensure(p, p->sub_off_i, sizeof(uint32_t) * (size_t)Ti));
 
-    std::vector<float> gscale(nt);
-    for (int g = 0; g < nt; ++g) {
-        const int64_t Mg = off[g + 1] - off[g];
-        gscale[g] = Mg > 0 ? (float)(1.0 / (double)Mg) : 0.f;
+    TileTotals *totals = p->counts.as<TileTotals>();
+    uint32_t *home_count = (uint32_t *)(totals + 1), *scount = home_count + Ti;
+    if (nt > 1 || M == 0) {
+        std::vector<float> gscale(nt);
+        for (int g = 0; g < nt; ++g) {
+            const int64_t Mg = off[g + 1] - off[g];
+            gscale[g] = Mg > 0 ? (float)(1.0 / (double)Mg) : 0.f;
+        }
+        GBN_CUDA(cudaMemcpyAsync(p->traj_off_d.p, off, sizeof(int64_t) * (nt + 1), cudaMemcpyHostToDevice, s));
+        GBN_CUDA(cudaMemcpyAsync(p->grp_scale.p, gscale.data(), sizeof(float) * nt, cudaMemcpyHostToDevice, s));
     }
-    GBN_CUDA(cudaMemcpyAsync(p->traj_off_d.p, off, sizeof(int64_t) * (nt + 1), cudaMemcpyHostToDevice, s));
-    GBN_CUDA(cudaMemcpyAsync(p->grp_scale.p, gscale.data(), sizeof(float) * nt, cudaMemcpyHostToDevice, s));
-    GBN_CUDA(cudaMemsetAsync(p->home_count.p, 0, sizeof(uint32_t) * (Ti + 1), s));
-    GBN_CUDA(cudaMemsetAsync(p->spread_count.p, 0, sizeof(uint32_t) * Ts, s));
+    GBN_CUDA(cudaMemsetAsync(totals, 0, count_bytes, s));
 
-    uint32_t *home_count = p->home_count.as<uint32_t>();
-    GBN_CUDA(launch_prep(dtype, x, y, z, M, p->traj_off_d.as<int64_t>(), p->gs, p->gi, p->desc.df,
-                         p->pts.as<float4>(), p->home_key.as<uint32_t>(), p->touch_count.as<uint32_t>(),
-                         home_count, s));
+    PrepArgs pa{};
+    pa.x = x;
+    pa.y = y;
+    pa.z = z;
+    pa.M = M;
+    pa.df = p->desc.df;
+    pa.gs = p->gs;
+    pa.gi = p->gi;
+    pa.scale1 = M > 0 ? (float)(1.0 / (double)M) : 0.f;
+    pa.traj_off = p->traj_off_d.as<int64_t>();
+    pa.grp_scale = p->grp_scale.as<float>();
+    pa.pts = p->pts.as<float4>();
+    pa.iota = p->iota.as<uint32_t>();
+    pa.home_key = p->home_key.as<uint32_t>();
+    pa.touch_count = p->touch_count.as<uint32_t>();
+    pa.home_count = home_count;
+    pa.tile_count = scount;
+    pa.status = &totals->status;
+    GBN_CUDA(launch_prep(dtype, pa, s));
+
+    // 3-D: spread tiles with at least dense_min samples (the k-space centre of radial
+    // trajectories) accumulate with compensated sums
+    const uint32_t dense_min = p->dim == 3 && p->dense_min > 0 ? (uint32_t)p->dense_min : 0u;
+    // the plane-streaming 3-D interp holds a chunk of kPlaneSamples samples' state; work
+    // items of at most that size stream each window once
+    const int interp_max_sub = interp3d_planes_smem(p->gi, interp_cg(p), p->interp_threads) > 0
+                                   ? std::min(p->max_sub, kPlaneSamples)
+                                   : std::min(p->max_sub, p->interp_max_sub);
+    p->spread_items_interleaved = spread_interleaved(p);
+    SubsJob js{}, ji{};
+    js.count = scount;
+    js.tile_off = p->spread_tile_off.as<uint32_t>();
+    js.sub_off = p->sub_off.as<uint32_t>();
+    js.T = Ts;
+    js.max_sub = p->max_sub;
+    js.every_tile = 1;
+    js.interleave = p->spread_items_interleaved ? 1 : 0;
+    js.dense_min = dense_min;
+    ji.count = home_count;
+    ji.tile_off = p->home_tile_off.as<uint32_t>();
+    ji.sub_off = p->sub_off_i.as<uint32_t>();
+    ji.T = Ti;
+    ji.max_sub = interp_max_sub;
+    GBN_CUDA(launch_tile_scan(js, ji, totals, s));
+
     uint32_t *tc = p->touch_count.as<uint32_t>();
     uint64_t *to = p->touch_off.as<uint64_t>();
     if (M > 0) {
@@ -679,62 +674,44 @@ int set_points_impl(gbn_plan *p, int dtype, const void *x, const void *y, const 
     }
     // The spread list (one entry per sample and tile its stencil reaches) has E = sum of the
     // touch counts entries.  When a bound on E fits kOneSyncEntries, its keys are written
-    // before E is known and the work-item counts are queued behind them, so one host
-    // synchronisation returns E, the counts and the status together (set_points on a changing
-    // trajectory, as in a differentiable reconstruction, then costs one round trip).  Per axis
-    // a W-cell stencil reaches at most ceil((W-1)/T) + 1 tiles, one more when a partial last
-    // tile sits at the wrap, and never more than the axis has.
+    // before E is known on the host, beside the home sort, so the round trip that brings E and
+    // the work-item counts back waits on no idle GPU.  Per axis a W-cell stencil reaches at
+    // most ceil((W-1)/T) + 1 tiles, one more when a partial last tile sits at the wrap, and
+    // never more than the axis has.
     uint64_t bound = (uint64_t)M;
     for (int d = 0; d < p->dim; ++d) {
         const Geom &g = p->gs;
         const uint64_t per = (uint64_t)((g.W - 1 + g.tile[d] - 1) / g.tile[d] + (g.nf[d] % g.tile[d] ? 2 : 1));
         bound *= std::min<uint64_t>(per, (uint64_t)g.ntile[d]);
     }
-    const bool one_sync = M > 0 && bound <= kOneSyncEntries;
-    uint32_t *scount = p->spread_count.as<uint32_t>();
-    // 3-D: spread tiles with at least dense_min samples (the k-space centre of radial
-    // trajectories) accumulate with compensated sums; status word 1 counts their work items,
-    // word 2 the split tiles (zeroed before each spread), word 3 is the split list's cursor
-    const uint32_t dense_min = p->dim == 3 && p->dense_min > 0 ? (uint32_t)p->dense_min : 0u;
-    GBN_TRY(ensure(p, p->split_tiles, sizeof(uint32_t) * (size_t)std::max<int64_t>(Ts, 1)));
-    // the plane-streaming 3-D interp holds a chunk of kPlaneSamples samples' state; work
-    // items of at most that size stream each window once
-    const int interp_max_sub = interp3d_planes_smem(p->gi, interp_cg(p), p->interp_threads) > 0
-                                   ? std::min(p->max_sub, kPlaneSamples)
-                                   : std::min(p->max_sub, p->interp_max_sub);
-    SubsJob js{&p->gs, scount, &p->spread_tile_off, &p->nsub, &p->sub_off, 1, p->max_sub, dense_min,
-               p->kstatus + 1, p->kstatus + 2};
-    js.interleave = spread_interleaved(p) ? 1 : 0;
-    p->spread_items_interleaved = js.interleave != 0;
-    SubsJob ji{&p->gi, home_count, &p->home_tile_off, &p->nsub_i, &p->sub_off_i, 0, interp_max_sub, 0u, nullptr,
-               nullptr};
-    uint32_t sizes[6] = {0, 0, 0, 0, 0, 0};  // spread last offset / count, interp ditto, dense, split
-    auto queue_counts = [&]() -> int {
-        GBN_CUDA(cudaMemsetAsync(p->kstatus + 1, 0, 4 * sizeof(uint32_t), s));
-        GBN_TRY(subs_count(p, js, sizes, s));
-        GBN_TRY(subs_count(p, ji, sizes + 2, s));
-        GBN_CUDA(cudaMemcpyAsync(sizes + 4, p->kstatus + 1, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    const bool early = M > 0 && bound <= kOneSyncEntries;
+    auto dup_keys = [&]() -> int {
+        GBN_CUDA(launch_dup_keys(p->pts.as<float4>(), M, p->traj_off_d.as<int64_t>(), p->gs, to,
+                                 p->dup_keys.as<uint32_t>(), p->dup_vals.as<uint32_t>(), s));
         return GBN_OK;
     };
-    if (one_sync) {
+    if (early) {
         GBN_TRY(ensure(p, p->dup_keys, sizeof(uint32_t) * (size_t)bound));
         GBN_TRY(ensure(p, p->dup_vals, sizeof(uint32_t) * (size_t)bound));
-        GBN_CUDA(launch_dup_keys(p->pts.as<float4>(), M, p->traj_off_d.as<int64_t>(), nt, p->gs, to,
-                                 p->dup_keys.as<uint32_t>(), p->dup_vals.as<uint32_t>(), scount, s));
-        GBN_TRY(queue_counts());
+        GBN_TRY(dup_keys());
     }
-    uint64_t last_off = 0;
-    uint32_t last_cnt = 0, status = 0;
     if (M > 0) {
-        GBN_CUDA(cudaMemcpyAsync(&last_off, to + (M - 1), sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-        GBN_CUDA(cudaMemcpyAsync(&last_cnt, tc + (M - 1), sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        uint32_t *kin = p->home_key.as<uint32_t>(), *vin = p->iota.as<uint32_t>();
+        uint32_t *kout = p->home_keys_sorted.as<uint32_t>(), *vout = p->home_idx.as<uint32_t>();
+        const int bits = key_bits((uint64_t)Ti);
+        GBN_TRY(cub_call(p, [&](void *tmp, size_t &bytes) {
+            return cub::DeviceRadixSort::SortPairs(tmp, bytes, kin, kout, vin, vout, (int)M, 0, bits, s);
+        }));
     }
-    GBN_CUDA(cudaMemcpyAsync(&status, home_count + Ti, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    TileTotals tot;
+    GBN_CUDA(cudaMemcpyAsync(&tot, totals, sizeof(tot), cudaMemcpyDeviceToHost, s));
     GBN_CUDA(cudaStreamSynchronize(s));
-    if (status & 1u) return fail(GBN_ERR_ARG, "non-finite trajectory coordinate");
-    const uint64_t E = M > 0 ? last_off + last_cnt : 0;
+    if (tot.status & 1u) return fail(GBN_ERR_ARG, "non-finite trajectory coordinate");
+    const uint64_t E = tot.entries;
     if (E >= ((uint64_t)1 << 31)) return fail(GBN_ERR_CAPACITY, "spread list above 2^31 entries");
-    if (one_sync && E > bound) return fail(GBN_ERR_INTERNAL, "spread list above its bound");
+    if (early && E > bound) return fail(GBN_ERR_INTERNAL, "spread list above its bound");
+    if (tot.spread_subs > 0x7FFFFFFF || tot.interp_subs > 0x7FFFFFFF)
+        return fail(GBN_ERR_CAPACITY, "too many subproblems");
     p->n_dup = (int64_t)E;
     const size_t Eb = (size_t)std::max<uint64_t>(E, 1);
     GBN_TRY(ensure(p, p->dup_keys, sizeof(uint32_t) * Eb));
@@ -742,9 +719,10 @@ int set_points_impl(gbn_plan *p, int dtype, const void *x, const void *y, const 
     GBN_TRY(ensure(p, p->dup_keys_sorted, sizeof(uint32_t) * Eb));
     GBN_TRY(ensure(p, p->dup_idx, sizeof(uint32_t) * Eb));
     GBN_TRY(ensure(p, p->dup_pts, sizeof(float4) * Eb));
-    if (!one_sync)
-        GBN_CUDA(launch_dup_keys(p->pts.as<float4>(), M, p->traj_off_d.as<int64_t>(), nt, p->gs, to,
-                                 p->dup_keys.as<uint32_t>(), p->dup_vals.as<uint32_t>(), scount, s));
+    GBN_TRY(ensure(p, p->spread_subs, sizeof(int4) * (size_t)std::max<uint64_t>(tot.spread_subs, 1)));
+    GBN_TRY(ensure(p, p->interp_subs, sizeof(int4) * (size_t)std::max<uint64_t>(tot.interp_subs, 1)));
+    GBN_TRY(ensure(p, p->dense_subs, sizeof(uint32_t) * (size_t)std::max<uint32_t>(tot.n_dense, 1)));
+    if (!early && M > 0) GBN_TRY(dup_keys());
     if (E > 0) {
         uint32_t *kin = p->dup_keys.as<uint32_t>(), *vin = p->dup_vals.as<uint32_t>();
         uint32_t *kout = p->dup_keys_sorted.as<uint32_t>(), *vout = p->dup_idx.as<uint32_t>();
@@ -752,30 +730,20 @@ int set_points_impl(gbn_plan *p, int dtype, const void *x, const void *y, const 
         GBN_TRY(cub_call(p, [&](void *tmp, size_t &bytes) {
             return cub::DeviceRadixSort::SortPairs(tmp, bytes, kin, kout, vin, vout, (int)E, 0, bits, s);
         }));
-        GBN_CUDA(launch_gather_pts(p->pts.as<float4>(), vout, (int64_t)E, p->dup_pts.as<float4>(), s));
     }
-    if (M > 0) {
-        k_iota<<<(unsigned)((M + 255) / 256), 256, 0, s>>>(p->iota.as<uint32_t>(), M);
-        GBN_CUDA(cudaGetLastError());
-        uint32_t *kin = p->home_key.as<uint32_t>(), *vin = p->iota.as<uint32_t>();
-        uint32_t *kout = p->home_keys_sorted.as<uint32_t>(), *vout = p->home_idx.as<uint32_t>();
-        const int bits = key_bits((uint64_t)Ti);
-        GBN_TRY(cub_call(p, [&](void *tmp, size_t &bytes) {
-            return cub::DeviceRadixSort::SortPairs(tmp, bytes, kin, kout, vin, vout, (int)M, 0, bits, s);
-        }));
-        GBN_CUDA(launch_gather_pts(p->pts.as<float4>(), vout, M, p->home_pts.as<float4>(), s));
-    }
-    if (!one_sync) {
-        GBN_TRY(queue_counts());
-        GBN_CUDA(cudaStreamSynchronize(s));
-    }
-    GBN_TRY(ensure(p, p->dense_subs, sizeof(uint32_t) * (size_t)std::max<uint32_t>(sizes[4], 1)));
-    GBN_TRY(subs_build(p, js, sizes, p->spread_subs, p->split_tiles.as<uint32_t>(), p->kstatus + 3,
-                       p->dense_subs.as<uint32_t>(), p->kstatus + 4, &p->n_spread_sub, s));
-    GBN_TRY(subs_build(p, ji, sizes + 2, p->interp_subs, nullptr, nullptr, nullptr, nullptr, &p->n_interp_sub, s));
-    const uint32_t counts[2] = {sizes[4], sizes[5]};
-    p->n_dense_sub = counts[0];
-    p->n_split = counts[1];
+    GBN_CUDA(launch_gather_pts(p->pts.as<float4>(), p->dup_idx.as<uint32_t>(), (int64_t)E, p->dup_pts.as<float4>(),
+                               p->home_idx.as<uint32_t>(), M, p->home_pts.as<float4>(), s));
+    js.split_list = p->split_tiles.as<uint32_t>();
+    js.split_cursor = &totals->split_cursor;
+    js.dense_list = p->dense_subs.as<uint32_t>();
+    js.dense_cursor = &totals->dense_cursor;
+    js.subs = p->spread_subs.as<int4>();
+    ji.subs = p->interp_subs.as<int4>();
+    GBN_CUDA(launch_build_subs(js, ji, s));
+    p->n_spread_sub = (int64_t)tot.spread_subs;
+    p->n_interp_sub = (int64_t)tot.interp_subs;
+    p->n_dense_sub = tot.n_dense;
+    p->n_split = tot.n_split;
     p->points_gen += 1;
     p->points_set = true;
     return GBN_OK;
@@ -1062,9 +1030,6 @@ int plan_create_impl(const gbn_plan_desc *desc, gbn_plan **out) {
         }
         p->device_bytes += sizeof(float) * p->m[d];
     }
-    // word 0: kernel status bits; words 1, 2: dense spread subproblems and split spread
-    // tiles (counted by set_points); words 3, 4: the cursors of the split-tile and
-    // dense-subproblem lists
     e = cudaMalloc((void **)&p->kstatus, 8 * sizeof(uint32_t));
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -1153,9 +1118,9 @@ int gbn_plan_destroy(gbn_plan *p) {
     for (int d = 0; d < 3; ++d)
         if (p->tab[d]) cudaFree(p->tab[d]);
     DevBuf *bufs[] = {&p->traj_off_d, &p->grp_scale, &p->pts, &p->home_key, &p->home_keys_sorted,
-                      &p->touch_count, &p->touch_off, &p->home_count, &p->iota, &p->home_idx, &p->home_pts,
+                      &p->touch_count, &p->touch_off, &p->counts, &p->iota, &p->home_idx, &p->home_pts,
                       &p->dup_keys, &p->dup_vals, &p->dup_keys_sorted, &p->dup_idx, &p->dup_pts,
-                      &p->spread_count, &p->spread_tile_off, &p->home_tile_off, &p->nsub, &p->sub_off, &p->nsub_i, &p->sub_off_i,
+                      &p->spread_tile_off, &p->home_tile_off, &p->sub_off, &p->sub_off_i,
                       &p->spread_subs, &p->interp_subs, &p->cub_tmp, &p->scratch, &p->stage_in,
                       &p->stage_out, &p->stage_w, &p->split_tiles, &p->dense_subs, &p->solve_ws, &p->dcf_ws};
     for (gbn_plan::SolveGraph &sg : p->solve_graph)

@@ -98,29 +98,47 @@ struct SortBuffers;
 int record_error(int code, const char *msg);
 
 // prep.cu
-cudaError_t launch_prep(int coord_dtype, const void *x, const void *y, const void *z, int64_t M,
-                        const int64_t *d_traj_off, const Geom &gs, const Geom &gi, double df,
-                        float4 *pts, uint32_t *home_key, uint32_t *touch_count, uint32_t *home_count,
-                        cudaStream_t s);
-cudaError_t launch_dup_keys(const float4 *pts, int64_t M, const int64_t *d_traj_off, int n_traj,
-                            const Geom &gs, const uint64_t *touch_off, uint32_t *keys, uint32_t *vals,
-                            uint32_t *tile_count, cudaStream_t s);
-cudaError_t launch_gather_pts(const float4 *pts, const uint32_t *idx, int64_t n, float4 *out,
-                              cudaStream_t s);
-// dense_min > 0: subproblems of tiles with at least dense_min samples get kDenseFlag.
-// split_list (may be null): the indices of the tiles covered by more than one subproblem
-// are appended at *split_cursor (zeroed by the caller).
-// interleave: split tiles' items take every s-th entry (only for the 3-D cube spread)
-// dense_list (may be null): the indices of the items with kDenseFlag are appended at
-// *dense_cursor (zeroed by the caller), in no particular order.
-cudaError_t launch_build_subs(const uint32_t *count, const uint32_t *tile_off, const uint32_t *sub_off,
-                              int64_t ntiles_total, int max_sub, int every_tile, uint32_t dense_min, int interleave,
-                              uint32_t *split_list, uint32_t *split_cursor, uint32_t *dense_list,
-                              uint32_t *dense_cursor, int4 *subs, cudaStream_t s);
-// work items per tile; n_dense (may be null) accumulates the items of tiles with at least
-// dense_min samples, n_split (may be null) the tiles split over several items
-cudaError_t launch_count_subs(const uint32_t *count, int64_t n, int max_sub, int every_tile, uint32_t dense_min,
-                              uint32_t *n_sub, uint32_t *n_dense, uint32_t *n_split, cudaStream_t s);
+struct PrepArgs {
+    const void *x, *y, *z;  // coordinates, radians
+    int64_t M;
+    double df;
+    double h[3], rh[3];     // cell size 2 pi / nf and its reciprocal (set by launch_prep)
+    Geom gs, gi;            // the spread's and the interp's bins
+    float scale1;           // 1 / M: the group scale where there is one group
+    int64_t *traj_off;      // group offsets and scales (one group: written here)
+    float *grp_scale;
+    float4 *pts;
+    uint32_t *iota, *home_key, *touch_count;
+    uint32_t *home_count, *tile_count;  // zeroed: samples per interp bin, entries per spread tile
+    uint32_t *status;                   // zeroed: bit 0 set by a coordinate that is not finite
+};
+cudaError_t launch_prep(int coord_dtype, PrepArgs a, cudaStream_t s);
+cudaError_t launch_dup_keys(const float4 *pts, int64_t M, const int64_t *d_traj_off, const Geom &gs,
+                            const uint64_t *touch_off, uint32_t *keys, uint32_t *vals, cudaStream_t s);
+// out[i] = pts[idx[i]] for both lists
+cudaError_t launch_gather_pts(const float4 *pts, const uint32_t *idx, int64_t n, float4 *out, const uint32_t *idx2,
+                              int64_t n2, float4 *out2, cudaStream_t s);
+// Work items of one bin geometry.  dense_min > 0: the items of tiles with at least dense_min
+// samples get kDenseFlag.  split_list, dense_list (may be null): the tiles covered by more than
+// one item, and the items with kDenseFlag, appended at their zeroed cursors in no particular
+// order.  interleave: split tiles' items take every s-th entry (cube and tensor-core spread).
+struct SubsJob {
+    const uint32_t *count;         // samples per tile
+    uint32_t *tile_off, *sub_off;  // exclusive sums of the samples and the items
+    int64_t T;                     // tiles of all groups
+    int max_sub, every_tile, interleave;
+    uint32_t dense_min;
+    uint32_t *split_list, *split_cursor, *dense_list, *dense_cursor;
+    int4 *subs;
+};
+struct TileTotals {  // zeroed by the caller, with the counts
+    uint64_t entries, home_entries, spread_subs, interp_subs;
+    uint32_t n_dense, n_split;     // dense work items, split tiles (spread)
+    uint32_t status;               // bit 0: a coordinate is not finite
+    uint32_t split_cursor, dense_cursor, pad;
+};
+cudaError_t launch_tile_scan(const SubsJob &spread, const SubsJob &home, TileTotals *out, cudaStream_t s);
+cudaError_t launch_build_subs(const SubsJob &spread, const SubsJob &home, cudaStream_t s);
 
 // grid.cu
 struct SpreadArgs {

@@ -12,8 +12,8 @@ namespace {
 
 constexpr double kTwoPi = 6.283185307179586476925286766559;
 
-// Python float semantics of a % b and a // b for b > 0 (CPython float_rem /
-// float_floor_div), so that the nearest-cell choice matches the reference.
+// Python float semantics of a % b for b > 0 (CPython float_rem), so that the nearest-cell
+// choice matches the reference.
 __device__ inline double py_mod(double a, double b) {
     double m = fmod(a, b);
     if (m != 0.0) {
@@ -23,20 +23,6 @@ __device__ inline double py_mod(double a, double b) {
     }
     return m;
 }
-__device__ inline double py_floordiv(double a, double b) {
-    double m = fmod(a, b);
-    double div = (a - m) / b;
-    if (m != 0.0 && ((b < 0) != (m < 0))) div -= 1.0;
-    double fd;
-    if (div != 0.0) {
-        fd = floor(div);
-        if (div - fd > 0.5) fd += 1.0;
-    } else {
-        fd = copysign(0.0, a / b);
-    }
-    return fd;
-}
-
 __device__ inline int group_of(const int64_t *off, int n_traj, int64_t j) {
     int lo = 0, hi = n_traj;  // off[lo] <= j < off[hi]
     while (hi - lo > 1) {
@@ -46,16 +32,48 @@ __device__ inline int group_of(const int64_t *off, int n_traj, int64_t j) {
     return lo;
 }
 
+// The nearest-cell choice of one coordinate: n = floor(xi / h) and the in-cell fraction, with
+// xi = xs mod 2 pi, as Python's % and // give them.  FP64 runs at 1/64 of the FP32 rate here,
+// and fmod and the divisions of the general form above took 129 of the 571 us that 256,000
+// 3-D samples needed; within (-2 pi, 2 pi) the remainder is xs or xs + 2 pi (fmod is exact),
+// and n follows from an estimate and the exact remainder xi - n h (one fused multiply-add,
+// whose sign and size say whether the estimate was one off; Python's xi // h, (xi - xi % h) / h
+// rounded to the nearest whole number, is that n).  12 FP64 instructions an axis.
+__device__ __forceinline__ void nearest_cell(double xs, double h, double rh, bool wide, int &n, float &fr) {
+    double xi = xs;
+    if (xs < 0.0) xi = xs + kTwoPi;
+    if (!(xi >= 0.0 && xs < kTwoPi)) xi = py_mod(xs, kTwoPi);  // outside (-2 pi, 2 pi)
+    // `wide`: more cells than an FP32 estimate places within one
+    int64_t k = wide ? (int64_t)(xi * rh) : (int64_t)(int)((float)xi * (float)rh);
+    double r = fma(-(double)k, h, xi);
+    if (r < 0.0) {
+        k -= 1;
+    } else if (r >= h) {
+        k += 1;
+    }
+    n = (int)k;
+    fr = (float)((xi - h * (double)k) * rh);
+}
+
+// one counter per key, keys of adjacent lanes often equal (samples along a spoke share tiles,
+// and the k-space centre is one tile for all of them): one atomic per distinct key of a warp
+__device__ __forceinline__ void count_key(uint32_t *count, uint32_t key) {
+    const unsigned same = __match_any_sync(__activemask(), key);
+    if ((threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&count[key], (uint32_t)__popc(same));
+}
+
 template <typename T>
-__global__ void k_prep(const T *__restrict__ x, const T *__restrict__ y, const T *__restrict__ z,
-                       int64_t M, const int64_t *__restrict__ traj_off, Geom gs, Geom gi, double df,
-                       float4 *__restrict__ pts, uint32_t *__restrict__ home_key,
-                       uint32_t *__restrict__ touch_count, uint32_t *__restrict__ home_count,
-                       uint32_t *__restrict__ status) {
-    int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j >= M) return;
+__global__ void __launch_bounds__(256) k_prep(PrepArgs a) {
+    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (j == 0 && a.gs.n_traj == 1) {  // one group: its offsets and scale need no copy
+        a.traj_off[0] = 0;
+        a.traj_off[1] = a.M;
+        a.grp_scale[0] = a.scale1;
+    }
+    if (j >= a.M) return;
+    const Geom &gs = a.gs, &gi = a.gi;
     const int dim = gs.dim, ns = gs.ns;
-    const T *src[3] = {x, y, z};
+    const T *src[3] = {(const T *)a.x, (const T *)a.y, (const T *)a.z};
     float f[3] = {0.f, 0.f, 0.f};
     int c0[3] = {0, 0, 0};
     bool bad = false;
@@ -64,45 +82,55 @@ __global__ void k_prep(const T *__restrict__ x, const T *__restrict__ y, const T
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         if (d >= dim) continue;
-        double xs = (double)src[d][j] * df;
+        const double xs = (double)src[d][j] * a.df;
         if (!isfinite(xs)) { bad = true; continue; }
         const int nf = gs.nf[d];
-        const double h = kTwoPi / nf;
-        double xi = py_mod(xs, kTwoPi);
-        int64_t m = 1 + (int64_t)py_floordiv(xi, h);
-        double fr = (xi - h * (double)(m - 1)) / h;
-        f[d] = (float)fr;
-        int64_t first = (m - ns) % nf;
+        int n;
+        nearest_cell(xs, a.h[d], a.rh[d], nf > (1 << 20), n, f[d]);
+        int first = (1 + n - ns) % nf;
         if (first < 0) first += nf;
-        c0[d] = (int)first;
+        c0[d] = first;
     }
     if (bad) {
-        atomicOr(status, 1u);
+        atomicOr(a.status, 1u);
         for (int d = 0; d < 3; ++d) { f[d] = 0.f; c0[d] = 0; }
     }
-    pts[j] = make_float4(f[0], f[1], f[2], __uint_as_float(pack_cells(dim, c0[0], c0[1], c0[2])));
+    a.pts[j] = make_float4(f[0], f[1], f[2], __uint_as_float(pack_cells(dim, c0[0], c0[1], c0[2])));
+    a.iota[j] = (uint32_t)j;
 
-    const int g = group_of(traj_off, gs.n_traj, j);
-    int t[3] = {0, 0, 0};
-    uint32_t touch = 1;
+    const int g = gs.n_traj == 1 ? 0 : group_of(a.traj_off, gs.n_traj, j);
+    int t[3] = {0, 0, 0}, n[3] = {1, 1, 1}, t0[3] = {0, 0, 0};
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         if (d >= dim) continue;
         int cc = c0[d] + ns - 1;
         if (cc >= gi.nf[d]) cc -= gi.nf[d];
         t[d] = cc / gi.tile[d];
-        touch *= (uint32_t)touched_tiles(c0[d], gs.W, gs.nf[d], gs.tile[d], gs.ntile[d]);
+        n[d] = touched_tiles(c0[d], gs.W, gs.nf[d], gs.tile[d], gs.ntile[d]);
+        t0[d] = c0[d] / gs.tile[d];
     }
-    uint32_t key = (uint32_t)g * (uint32_t)gi.ntiles +
-                   (uint32_t)((t[0] * gi.ntile[1] + t[1]) * gi.ntile[2] + t[2]);
-    home_key[j] = key;
-    atomicAdd(&home_count[key], 1u);
-    touch_count[j] = touch;
+    const uint32_t key = (uint32_t)g * (uint32_t)gi.ntiles +
+                         (uint32_t)((t[0] * gi.ntile[1] + t[1]) * gi.ntile[2] + t[2]);
+    a.home_key[j] = key;
+    count_key(a.home_count, key);
+    a.touch_count[j] = (uint32_t)(n[0] * n[1] * n[2]);
+    const uint32_t base = (uint32_t)g * (uint32_t)gs.ntiles;
+    for (int p = 0; p < n[0]; ++p) {
+        const int tp = (t0[0] + p) % gs.ntile[0];
+        for (int b = 0; b < n[1]; ++b) {
+            const int tb = (t0[1] + b) % gs.ntile[1];
+            for (int q = 0; q < n[2]; ++q) {
+                const int tq = (t0[2] + q) % gs.ntile[2];
+                count_key(a.tile_count, base + (uint32_t)((tp * gs.ntile[1] + tb) * gs.ntile[2] + tq));
+            }
+        }
+    }
 }
 
+// the (sample, tile) entries, each sample's adjacent
 __global__ void k_dup_keys(const float4 *__restrict__ pts, int64_t M, const int64_t *__restrict__ traj_off,
                            Geom gs, const uint64_t *__restrict__ touch_off, uint32_t *__restrict__ keys,
-                           uint32_t *__restrict__ vals, uint32_t *__restrict__ tile_count) {
+                           uint32_t *__restrict__ vals) {
     int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (j >= M) return;
     const int dim = gs.dim;
@@ -115,7 +143,7 @@ __global__ void k_dup_keys(const float4 *__restrict__ pts, int64_t M, const int6
         n[d] = touched_tiles(c0[d], gs.W, gs.nf[d], gs.tile[d], gs.ntile[d]);
         t0[d] = c0[d] / gs.tile[d];
     }
-    const uint32_t base = (uint32_t)group_of(traj_off, gs.n_traj, j) * (uint32_t)gs.ntiles;
+    const uint32_t base = gs.n_traj == 1 ? 0u : (uint32_t)group_of(traj_off, gs.n_traj, j) * (uint32_t)gs.ntiles;
     uint64_t pos = touch_off[j];
     for (int a = 0; a < n[0]; ++a) {
         int ta = (t0[0] + a) % gs.ntile[0];
@@ -123,66 +151,133 @@ __global__ void k_dup_keys(const float4 *__restrict__ pts, int64_t M, const int6
             int tb = (t0[1] + b) % gs.ntile[1];
             for (int q = 0; q < n[2]; ++q) {
                 int tq = (t0[2] + q) % gs.ntile[2];
-                uint32_t key = base + (uint32_t)((ta * gs.ntile[1] + tb) * gs.ntile[2] + tq);
-                keys[pos] = key;
+                keys[pos] = base + (uint32_t)((ta * gs.ntile[1] + tb) * gs.ntile[2] + tq);
                 vals[pos] = (uint32_t)j;
-                atomicAdd(&tile_count[key], 1u);
                 ++pos;
             }
         }
     }
 }
 
+// records in list order, for both lists
 __global__ void k_gather_pts(const float4 *__restrict__ pts, const uint32_t *__restrict__ idx, int64_t n,
-                             float4 *__restrict__ out) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+                             float4 *__restrict__ out, const uint32_t *__restrict__ idx2, int64_t n2,
+                             float4 *__restrict__ out2) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i < n) out[i] = pts[idx[i]];
+    else if (i - n < n2) out2[i - n] = pts[idx2[i - n]];
 }
 
-// per tile: its number of work items; optionally counts the work items of dense tiles
-// (n_dense) and the tiles split over several items (n_split)
-__global__ void k_count_subs(const uint32_t *__restrict__ count, int64_t n, int max_sub, int every_tile,
-                             uint32_t dense_min, uint32_t *__restrict__ n_sub, uint32_t *n_dense,
-                             uint32_t *n_split) {
-    int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    uint32_t c = count[t];
-    uint32_t s = (c + (uint32_t)max_sub - 1) / (uint32_t)max_sub;
-    if (every_tile && s == 0) s = 1;
-    n_sub[t] = s;
-    if (n_dense && dense_min > 0 && c >= dense_min) atomicAdd(n_dense, s);
-    if (n_split && s > 1) atomicAdd(n_split, 1u);
+__device__ __forceinline__ uint32_t items_of(uint32_t c, const SubsJob &j) {
+    const uint32_t s = (c + (uint32_t)j.max_sub - 1) / (uint32_t)j.max_sub;
+    return j.every_tile && s == 0 ? 1u : s;
+}
+
+// Per tile, the exclusive sums of its entries (tile_off) and of its work items (sub_off), and
+// the totals.  One block per bin geometry walks its tiles 4096 at a time (1,024 to 37,000
+// tiles in the benchmark workloads): it stands for two device scans and a count kernel per
+// geometry, whose ten launches and separate read-backs took longer than the work.
+__global__ void __launch_bounds__(1024) k_tile_scan(SubsJob spread, SubsJob home, TileTotals *out) {
+    const SubsJob &j = blockIdx.x == 0 ? spread : home;
+    __shared__ uint64_t sh_c[32];
+    __shared__ uint32_t sh_s[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint64_t base_c = 0;
+    uint64_t base_s = 0;
+    uint32_t dense = 0, split = 0;
+    for (int64_t t0 = 0; t0 < j.T; t0 += 4096) {
+        const int64_t t = t0 + 4 * threadIdx.x;
+        uint32_t c[4], s[4];
+        uint64_t sum_c = 0;
+        uint32_t sum_s = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            c[i] = t + i < j.T ? j.count[t + i] : 0u;
+            s[i] = t + i < j.T ? items_of(c[i], j) : 0u;
+            if (j.dense_min > 0 && c[i] >= j.dense_min) dense += s[i];
+            if (s[i] > 1) split += 1;
+            sum_c += c[i];
+            sum_s += s[i];
+        }
+        uint64_t ic = sum_c;
+        uint32_t is = sum_s;
+#pragma unroll
+        for (int m = 1; m < 32; m <<= 1) {
+            const uint64_t vc = __shfl_up_sync(0xffffffffu, ic, m);
+            const uint32_t vs = __shfl_up_sync(0xffffffffu, is, m);
+            if (lane >= m) {
+                ic += vc;
+                is += vs;
+            }
+        }
+        if (lane == 31) {
+            sh_c[warp] = ic;
+            sh_s[warp] = is;
+        }
+        __syncthreads();
+        uint64_t wc = 0, tc = 0;
+        uint64_t ws = 0, ts = 0;
+#pragma unroll
+        for (int w = 0; w < 32; ++w) {
+            if (w < warp) {
+                wc += sh_c[w];
+                ws += sh_s[w];
+            }
+            tc += sh_c[w];
+            ts += sh_s[w];
+        }
+        uint64_t ec = base_c + wc + ic - sum_c;
+        uint64_t es = base_s + ws + is - sum_s;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (t + i < j.T) {
+                j.tile_off[t + i] = (uint32_t)ec;
+                j.sub_off[t + i] = (uint32_t)es;
+                ec += c[i];
+                es += s[i];
+            }
+        base_c += tc;
+        base_s += ts;
+        __syncthreads();  // sh_* are read
+    }
+    if (blockIdx.x == 0) {
+        dense = __reduce_add_sync(0xffffffffu, dense);
+        split = __reduce_add_sync(0xffffffffu, split);
+        if (lane == 0) {
+            atomicAdd(&out->n_dense, dense);
+            atomicAdd(&out->n_split, split);
+        }
+    }
+    if (threadIdx.x == 0) {
+        (blockIdx.x == 0 ? out->entries : out->home_entries) = base_c;
+        (blockIdx.x == 0 ? out->spread_subs : out->interp_subs) = base_s;
+    }
 }
 
 // interleave: the s > 1 items of a split tile take every s-th entry (item k: entries k,
 // k + s, k + 2s, ...; stride s in the flags above kStrideShift) instead of consecutive runs,
 // so that each item holds a spatially even share of the tile's samples
-__global__ void k_build_subs(const uint32_t *__restrict__ count, const uint32_t *__restrict__ tile_off,
-                             const uint32_t *__restrict__ sub_off, int64_t n, int max_sub, int every_tile,
-                             uint32_t dense_min, int interleave, uint32_t *__restrict__ split_list,
-                             uint32_t *__restrict__ split_cursor, uint32_t *__restrict__ dense_list,
-                             uint32_t *__restrict__ dense_cursor, int4 *__restrict__ subs) {
-    int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    uint32_t c = count[t];
-    uint32_t s = (c + (uint32_t)max_sub - 1) / (uint32_t)max_sub;
-    if (every_tile && s == 0) s = 1;
-    uint32_t o = sub_off[t];
-    const bool dense = dense_min > 0 && c >= dense_min;
-    if (s > 1 && split_list) split_list[atomicAdd(split_cursor, 1u)] = (uint32_t)t;  // order is irrelevant
-    if (dense && s > 0 && dense_list) {
-        const uint32_t d = atomicAdd(dense_cursor, s);
-        for (uint32_t k = 0; k < s; ++k) dense_list[d + k] = o + k;
+// (blockIdx.y 0: the spread's items, 1: the interp's)
+__global__ void k_build_subs(SubsJob spread, SubsJob home) {
+    const SubsJob &j = blockIdx.y == 0 ? spread : home;
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t >= j.T) return;
+    const uint32_t c = j.count[t], s = items_of(c, j), o = j.sub_off[t];
+    const bool dense = j.dense_min > 0 && c >= j.dense_min;
+    if (s > 1 && j.split_list) j.split_list[atomicAdd(j.split_cursor, 1u)] = (uint32_t)t;  // order is irrelevant
+    if (dense && s > 0 && j.dense_list) {
+        const uint32_t d = atomicAdd(j.dense_cursor, s);
+        for (uint32_t k = 0; k < s; ++k) j.dense_list[d + k] = o + k;
     }
     for (uint32_t k = 0; k < s; ++k) {
         int flags = (s > 1 ? kSplitFlag : 0) | (k == 0 ? kFirstFlag : 0) | (dense ? kDenseFlag : 0);
-        if (interleave && s > 1) {
+        if (j.interleave && s > 1) {
             const uint32_t len = (c - k + s - 1) / s;  // entries k, k + s, ... below c
-            subs[o + k] = make_int4((int)t, (int)(tile_off[t] + k), (int)len, flags | (int)(s << kStrideShift));
+            j.subs[o + k] = make_int4((int)t, (int)(j.tile_off[t] + k), (int)len, flags | (int)(s << kStrideShift));
         } else {
-            uint32_t start = k * (uint32_t)max_sub;
-            uint32_t len = c > start ? min((uint32_t)max_sub, c - start) : 0u;
-            subs[o + k] = make_int4((int)t, (int)(tile_off[t] + start), (int)len, flags);
+            const uint32_t start = k * (uint32_t)j.max_sub;
+            const uint32_t len = c > start ? min((uint32_t)j.max_sub, c - start) : 0u;
+            j.subs[o + k] = make_int4((int)t, (int)(j.tile_off[t] + start), (int)len, flags);
         }
     }
 }
@@ -191,56 +286,42 @@ inline unsigned blocks_for(int64_t n, int threads) { return (unsigned)((n + thre
 
 }  // namespace
 
-cudaError_t launch_prep(int coord_dtype, const void *x, const void *y, const void *z, int64_t M,
-                        const int64_t *d_traj_off, const Geom &gs, const Geom &gi, double df,
-                        float4 *pts, uint32_t *home_key, uint32_t *touch_count, uint32_t *home_count,
-                        cudaStream_t s) {
-    // status word lives right after home_count's last tile entry (allocated by the caller)
-    uint32_t *status = home_count + (size_t)gi.ntiles * gi.n_traj;
-    if (M == 0) return cudaSuccess;
-    const int th = 256;
+cudaError_t launch_prep(int coord_dtype, PrepArgs a, cudaStream_t s) {
+    if (a.M == 0) return cudaSuccess;
+    for (int d = 0; d < 3; ++d) {
+        a.h[d] = kTwoPi / a.gs.nf[d];
+        a.rh[d] = 1.0 / a.h[d];
+    }
     if (coord_dtype == GBN_COORD_F64)
-        k_prep<double><<<blocks_for(M, th), th, 0, s>>>((const double *)x, (const double *)y, (const double *)z,
-                                                      M, d_traj_off, gs, gi, df, pts, home_key, touch_count,
-                                                      home_count, status);
+        k_prep<double><<<blocks_for(a.M, 256), 256, 0, s>>>(a);
     else
-        k_prep<float><<<blocks_for(M, th), th, 0, s>>>((const float *)x, (const float *)y, (const float *)z,
-                                                     M, d_traj_off, gs, gi, df, pts, home_key, touch_count,
-                                                     home_count, status);
+        k_prep<float><<<blocks_for(a.M, 256), 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 
-cudaError_t launch_dup_keys(const float4 *pts, int64_t M, const int64_t *d_traj_off, int n_traj,
-                            const Geom &gs, const uint64_t *touch_off, uint32_t *keys, uint32_t *vals,
-                            uint32_t *tile_count, cudaStream_t s) {
-    (void)n_traj;
+cudaError_t launch_dup_keys(const float4 *pts, int64_t M, const int64_t *d_traj_off, const Geom &gs,
+                            const uint64_t *touch_off, uint32_t *keys, uint32_t *vals, cudaStream_t s) {
     if (M == 0) return cudaSuccess;
-    k_dup_keys<<<blocks_for(M, 256), 256, 0, s>>>(pts, M, d_traj_off, gs, touch_off, keys, vals, tile_count);
+    k_dup_keys<<<blocks_for(M, 256), 256, 0, s>>>(pts, M, d_traj_off, gs, touch_off, keys, vals);
     return cudaGetLastError();
 }
 
-cudaError_t launch_gather_pts(const float4 *pts, const uint32_t *idx, int64_t n, float4 *out, cudaStream_t s) {
-    if (n == 0) return cudaSuccess;
-    k_gather_pts<<<blocks_for(n, 256), 256, 0, s>>>(pts, idx, n, out);
+cudaError_t launch_gather_pts(const float4 *pts, const uint32_t *idx, int64_t n, float4 *out, const uint32_t *idx2,
+                              int64_t n2, float4 *out2, cudaStream_t s) {
+    if (n + n2 == 0) return cudaSuccess;
+    k_gather_pts<<<blocks_for(n + n2, 256), 256, 0, s>>>(pts, idx, n, out, idx2, n2, out2);
     return cudaGetLastError();
 }
 
-cudaError_t launch_count_subs(const uint32_t *count, int64_t n, int max_sub, int every_tile, uint32_t dense_min,
-                              uint32_t *n_sub, uint32_t *n_dense, uint32_t *n_split, cudaStream_t s) {
-    if (n == 0) return cudaSuccess;
-    k_count_subs<<<blocks_for(n, 256), 256, 0, s>>>(count, n, max_sub, every_tile, dense_min, n_sub, n_dense,
-                                                    n_split);
+cudaError_t launch_tile_scan(const SubsJob &spread, const SubsJob &home, TileTotals *out, cudaStream_t s) {
+    k_tile_scan<<<2, 1024, 0, s>>>(spread, home, out);
     return cudaGetLastError();
 }
 
-cudaError_t launch_build_subs(const uint32_t *count, const uint32_t *tile_off, const uint32_t *sub_off,
-                              int64_t ntiles_total, int max_sub, int every_tile, uint32_t dense_min, int interleave,
-                              uint32_t *split_list, uint32_t *split_cursor, uint32_t *dense_list,
-                              uint32_t *dense_cursor, int4 *subs, cudaStream_t s) {
-    if (ntiles_total == 0) return cudaSuccess;
-    k_build_subs<<<blocks_for(ntiles_total, 256), 256, 0, s>>>(count, tile_off, sub_off, ntiles_total, max_sub,
-                                                               every_tile, dense_min, interleave, split_list,
-                                                               split_cursor, dense_list, dense_cursor, subs);
+cudaError_t launch_build_subs(const SubsJob &spread, const SubsJob &home, cudaStream_t s) {
+    const int64_t T = spread.T > home.T ? spread.T : home.T;
+    if (T == 0) return cudaSuccess;
+    k_build_subs<<<dim3(blocks_for(T, 256), 2), 256, 0, s>>>(spread, home);
     return cudaGetLastError();
 }
 
