@@ -106,6 +106,14 @@ __global__ void __launch_bounds__(512) k_interp2d_tma(InterpArgs a, const __grid
     for (int64_t item = blockIdx.x; item < t.n_items; item += stride, b = (b + 1 == S) ? 0 : b + 1) {
         float2 *win = bufs + (size_t)b * t.buf_elems;
         const TmaItem it = ring[b];
+        // the first records' loads overlap the wait for the window
+        const int4 sub = it.sub;
+        float4 p_next = make_float4(0.f, 0.f, 0.f, 0.f);
+        uint32_t j_next = 0;
+        if (warp < sub.z) {
+            p_next = a.pts[(int64_t)sub.y + warp];
+            j_next = a.idx[(int64_t)sub.y + warp];
+        }
         int off1 = 0;
         if (it.tma) {
             if (!mbar_wait_bounded(&bar[b], (parity >> b) & 1u) && lane == 0) atomicOr(status, kStatusTmaTimeout);
@@ -127,13 +135,6 @@ __global__ void __launch_bounds__(512) k_interp2d_tma(InterpArgs a, const __grid
             __syncthreads();
         }
 
-        const int4 sub = it.sub;
-        float4 p_next = make_float4(0.f, 0.f, 0.f, 0.f);
-        uint32_t j_next = 0;
-        if (warp < sub.z) {
-            p_next = a.pts[(int64_t)sub.y + warp];
-            j_next = a.idx[(int64_t)sub.y + warp];
-        }
         for (int s = warp; s < sub.z; s += nw) {
             const float4 p = p_next;
             const uint32_t j = j_next;
@@ -150,7 +151,7 @@ __global__ void __launch_bounds__(512) k_interp2d_tma(InterpArgs a, const __grid
             float myw = 0.f;
             if (kk < W) {
                 const float d = (lane < 16 ? p.x : p.y) + (float)(ns - 1 - kk);
-                myw = exp2f(-beta * d * d);
+                myw = ex2_approx(-beta * d * d);
             }
             float wy[L::KT];
 #pragma unroll
