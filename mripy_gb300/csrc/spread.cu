@@ -133,7 +133,7 @@ static cudaError_t launch_cube(const SpreadArgs &a, int64_t n_sub, cudaStream_t 
 template <int WT, bool KAHAN>
 static cudaError_t launch_mma_instance(const SpreadArgs &a, int64_t n_units, int n_cg, cudaStream_t s) {
     auto kern = k_spread_mma<3, WT, KAHAN>;
-    const size_t smem = KAHAN ? kMmaSmemBytesK : kMmaSmemBytes;
+    constexpr size_t smem = MmaCfg<3, KAHAN>::SMEM;
     cudaError_t e = set_smem(kern, smem);
     if (e != cudaSuccess) return e;
     // the compensated instance: one block per (dense subproblem, coil group) only
@@ -149,9 +149,9 @@ static cudaError_t launch_mma(const SpreadArgs &a, int64_t n_sub, cudaStream_t s
     const int64_t n_units = n_sub * n_cg;
     if (a.g.dim == 2) {  // no dense tiles in 2-D
         auto kern = k_spread_mma<2, WT, false>;
-        cudaError_t e = set_smem(kern, kMmaSmemBytes);
+        cudaError_t e = set_smem(kern, MmaCfg<2, false>::SMEM);
         if (e != cudaSuccess) return e;
-        kern<<<(unsigned)n_units, mma_threads<false>(), kMmaSmemBytes, s>>>(a, a.status, n_cg);
+        kern<<<(unsigned)n_units, mma_threads<false>(), MmaCfg<2, false>::SMEM, s>>>(a, a.status, n_cg);
         return cudaGetLastError();
     }
     cudaError_t e = launch_mma_instance<WT, false>(a, n_units, n_cg, s);

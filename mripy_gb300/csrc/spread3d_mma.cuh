@@ -20,24 +20,31 @@
 //
 // One (work item, coil group) unit per block; 3 loader warps, NB builder warps (8 in the
 // plain instance, 16 in the compensated one) and 1 MMA warp:
-// * the loader warps fill a ring of kMmaSlots 32-sample batches (loader l: batches l, l + 3,
-//   ...; the sample indices of batch l are read before the block's set-up): per sample and
-//   dimension the first tap's tile plane and the distance of plane 0, and the 8 coil values
-//   times the optional density weight ([coil][sample]); `full` / `empty` mbarriers per slot.
-// * the builder warps first compute the batch's tile-plane weights per sample together
-//   (stored [plane][sample]; a named barrier among them), then turn the batch into the MMA
-//   operands: warp b writes A's hi and lo parts for the 32 TMEM lanes of its quarter (b % 4)
-//   and 128 / NB of the 32 samples, and N / NB of B's rows into shared memory; two operand
-//   buffers, the one of batch t reused by batch t + 2 after the MMAs of batch t completed
-//   (`done` mbarrier, signalled by tcgen05.commit).  After the last batch they read D back
-//   (tcgen05.ld) and write the tile.
+// * the loader warps fill a ring of 32-sample batches (loader l: batches l, l + 3, ...; the
+//   sample indices of batch l are read before the block's set-up): per sample its tile-plane
+//   weights ([plane][sample]) and the 8 coil values times the optional density weight
+//   ([coil][sample]); `full` / `empty` mbarriers per slot.
+// * the builder warps turn a batch into the MMA operands: a warp writes A's hi and lo parts
+//   for the 32 TMEM lanes of its quarter and its share of the samples, and its share of B's
+//   rows into shared memory; the operand buffer of batch t is reused by batch t + BUFS after
+//   the MMAs of batch t completed (`done` mbarrier, signalled by tcgen05.commit).  In the
+//   plain 3-D instance two groups of 4 warps build alternate batches, so that one group's
+//   waits, fences and loads overlap the other's building.  After the last batch they read D
+//   back (tcgen05.ld) and write the tile.
 // * the MMA warp allocates TMEM, and its lane 0 issues 12 MMAs per batch once the builders
 //   arrived on the buffer's `ops` mbarrier, then commits to the buffer's `done` mbarrier.
+//
+// What bounds it: the chain of waits per batch and the instructions of building, not the
+// tensor pipe (36 % active).  2.56 M samples x 8 coils on 256^3, 12 taps, with the compensated
+// instance: 5.36 ms with the weights computed by the builders behind a barrier of their own;
+// 4.45 with the weights in the loaders; 4.12 with three operand buffers, two builder groups and
+// 16-byte coil loads.  (16 builder warps: 4.94; 4 in one group: 4.69; 2 or 4 loaders: 4.98,
+// 4.60; loaders prefetching a batch ahead: 4.51.)
 // Summation: the tensor core's FP32 accumulation rounds less carefully than FP32 adds (its
 // error grew with the number of accumulated MMAs: 1.6e-6 relative to the FP32 kernel with
 // 1024-sample work items, 4.9e-6 with 8192, on the 3-D radial workload), so the plain
 // instance sums groups of kMmaGroup batches (256 samples, 96 MMAs) only; the builders then
-// add the accumulator into a running sum S in TMEM with FP32 adds before the next group's
+// add the accumulator into a running sum S (3-D: shared memory) with FP32 adds before the next group's
 // first MMA overwrites it.  The compensated instance (KAHAN: the 3-D dense, k-space-centre
 // units, one block per SM) drains every batch's accumulator (two of them alternate) into a
 // group sum G with FP32 adds and folds G into a Kahan-compensated sum S, C in TMEM every
@@ -62,14 +69,13 @@ constexpr int kMmaTX = 4, kMmaTY = 8, kMmaTZ = 16;  // the tile this kernel take
 constexpr int kMmaM = kMmaTY * kMmaTZ;              // 128 cells (y, z): one TMEM lane each
 constexpr int kMmaN = kMmaTX * 16;                  // 64 columns (x, coil, re/im)
 constexpr int kMmaBatch = 32;                       // samples per batch: one 128-byte K row
-constexpr int kMmaSlots = 8;                        // staged batches
-#ifndef GBN_MMA_LOADERS
-#define GBN_MMA_LOADERS 3
-#endif
-constexpr int kMmaLoaders = GBN_MMA_LOADERS;
+constexpr int kMmaLoaders = 3;
 // builder warps: 8 in the plain instance (two blocks per SM, registers), 16 in the
 // compensated one (one block per SM: more warps hide its latencies)
 template <bool KAHAN> constexpr int mma_builders() { return KAHAN ? 16 : 8; }
+// The plain 3-D instance's builders work as two groups of 4 warps on alternate batches, each
+// with its own operand buffer
+template <int D, bool KAHAN> constexpr int mma_groups() { return D == 3 && !KAHAN ? 2 : 1; }
 template <bool KAHAN> constexpr int mma_threads() { return 32 * (mma_builders<KAHAN>() + kMmaLoaders + 1); }
 constexpr uint32_t kMmaTmemCols = 256;              // A (hi, lo) x 2 buffers: 0..127; D, S: 128..255
 constexpr uint32_t kMmaColD = 128;                  // the MMAs' accumulator
@@ -86,23 +92,33 @@ constexpr uint32_t kMmaBOp = kMmaN * 128;                               // one B
 constexpr uint32_t kMmaStWx = 0;                                        // [TX][kMmaWS] floats
 constexpr uint32_t kMmaStWy = kMmaStWx + 4 * kMmaTX * kMmaWS;           // [TY][kMmaWS]
 constexpr uint32_t kMmaStWz = kMmaStWy + 4 * kMmaTY * kMmaWS;           // [TZ][kMmaWS]
-constexpr uint32_t kMmaStV = kMmaStWz + 4 * kMmaTZ * kMmaWS;            // [8 coils][32] float2
-constexpr uint32_t kMmaStD0 = kMmaStV + 8 * 8 * kMmaBatch;              // [3][32] float: d of tap 0
-constexpr uint32_t kMmaStR = kMmaStD0 + 4 * 3 * kMmaBatch;              // [3][32] int: first tap's cell
-constexpr uint32_t kMmaSlotBytes = kMmaStR + 4 * 3 * kMmaBatch;
-constexpr uint32_t kMmaStageOff = 4 * kMmaBOp;                          // after B (hi, lo) x 2 buffers
-constexpr uint32_t kMmaBarOff = kMmaStageOff + kMmaSlots * kMmaSlotBytes;
-constexpr uint32_t kMmaBars = 2 * kMmaSlots + 4;                        // full, empty, ops[2], done[2]
-// + the TMEM address word and the alignment slack.  Above a third of the SM's 228 KB, so at
-// most two blocks (2 x 256 TMEM columns) share an SM and tcgen05.alloc never waits.
-constexpr size_t kMmaSmemBytes = kMmaBarOff + 8 * kMmaBars + 16 + 1024;
-static_assert(kMmaSmemBytes > 228 * 1024 / 3, "two blocks per SM at most");
-// the compensated instance asks for more than half the SM's shared memory: one block per SM
-// holds all 512 TMEM columns
-constexpr size_t kMmaSmemBytesK = 116 * 1024;
-static_assert(kMmaSmemBytesK > 228 * 1024 / 2 && kMmaSmemBytesK >= kMmaSmemBytes, "one block per SM");
+constexpr int kMmaVS = kMmaBatch + 2;  // float2 per staged coil row: the four 16-byte quarters of a
+                                       // sample's coils are stored to distinct banks
+constexpr uint32_t kMmaStV = kMmaStWz + 4 * kMmaTZ * kMmaWS;            // [8 coils][kMmaVS] float2
+constexpr uint32_t kMmaSlotBytes = kMmaStV + 8 * 8 * kMmaVS;
 static_assert(kMmaStV % 16 == 0 && kMmaSlotBytes % 16 == 0, "16-byte aligned staging");
-constexpr int kMmaTaps = kMmaTX + kMmaTY + kMmaTZ;  // 28 tile-plane weights per sample
+// Per instance: operand buffers, staged batches, and the offsets after B's buffers.  The plain
+// 3-D instance keeps three operand buffers -- A's third one takes the TMEM columns of the
+// running sum S, which lives in shared memory there -- because a batch's chain (build, MMAs,
+// commit, next build) takes longer than two batches of building: 8 % of its time.
+template <int D, bool KAHAN> struct MmaCfg {
+    static constexpr int BUFS = D == 3 && !KAHAN ? 3 : 2;
+    static constexpr int SLOTS = D == 3 && !KAHAN ? 5 : 8;
+    static constexpr uint32_t STAGE = 2 * BUFS * kMmaBOp;                 // B (hi, lo) x BUFS
+    static constexpr uint32_t SUM = STAGE + SLOTS * kMmaSlotBytes;        // S: [64 columns][128 lanes] floats
+    static constexpr uint32_t BAR = SUM + (BUFS == 3 ? 4 * kMmaN * kMmaM : 0);
+    static constexpr uint32_t BARS = 2 * SLOTS + 2 * BUFS;                // full, empty, ops, done
+    // + the TMEM address word and the alignment slack
+    static constexpr size_t NEED = BAR + 8 * BARS + 16 + 1024;
+    // The compensated instance asks for more than half the SM's shared memory: one block per SM
+    // holds all 512 TMEM columns.  The others take more than a third, so at most two blocks
+    // (2 x 256 TMEM columns) share an SM and tcgen05.alloc never waits.
+    static constexpr size_t SMEM = KAHAN ? 116 * 1024 : (NEED > 77 * 1024 ? NEED : 77 * 1024);
+    static_assert(SMEM >= NEED && SMEM > 228 * 1024 / 3, "shared memory");
+    static_assert(KAHAN ? SMEM > 228 * 1024 / 2 : 2 * (SMEM + 1024) <= 228 * 1024, "blocks per SM");
+    // A's TMEM columns of buffer b
+    static __device__ __forceinline__ uint32_t a_col(int b) { return BUFS == 3 && b == 2 ? 192u : 64u * b; }
+};
 
 // The tile of each dimension: M = TY x TZ = 128 cells of grid dimensions (DY, DZ), N = NX
 // planes along grid dimension 0 (3-D only) x 8 coils x re/im.  3-D: 4 x 8 x 16 cells,
@@ -137,24 +153,22 @@ __device__ __forceinline__ void tf32_split2(float2 a, float2 b, float2 &hi, floa
 
 // S (+)= D over this thread's lane and the N / 2 columns of half hk; `first`: S = D.  D is
 // at column kMmaColD, S right after it (N columns each).
-template <int N>
-__device__ __forceinline__ void mma_drain(uint32_t tl, int hk, bool first) {
+// Where ssum is given (3-D), S is kept there: [column][128 lanes], this lane's at ssum.
+template <int N, int DPW>
+__device__ __forceinline__ void mma_drain(uint32_t tl, int hk, bool first, float *ssum = nullptr) {
     constexpr uint32_t kColS = kMmaColD + N;
     if constexpr (N == 64) {
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t col = 32u * hk + 16u * h;
-            float d[16], s[16];
+        for (int h = 0; h < DPW / 16; ++h) {
+            const uint32_t col = (uint32_t)DPW * hk + 16u * h;
+            float d[16];
             tmem_ld_x16(tl + kMmaColD + col, d);
-            if (!first) {
-                tmem_ld_x16(tl + kColS + col, s);
-                tmem_wait_ld();
+            tmem_wait_ld();
 #pragma unroll
-                for (int i = 0; i < 16; ++i) d[i] += s[i];
-            } else {
-                tmem_wait_ld();
+            for (int i = 0; i < 16; ++i) {
+                float &t = ssum[(col + i) * kMmaM];
+                t = first ? d[i] : t + d[i];
             }
-            tmem_st_x16(tl + kColS + col, d);
         }
     } else {
         static_assert(N == 16, "N is 64 (3-D) or 16 (2-D)");
@@ -244,9 +258,12 @@ template <int D, int WT, bool KAHAN>
 __global__ void __launch_bounds__(mma_threads<KAHAN>(), KAHAN ? 1 : 2) k_spread_mma(SpreadArgs a, uint32_t *status, int n_cg) {
     constexpr int NB = mma_builders<KAHAN>();  // builder warps
     constexpr int WM = NB + kMmaLoaders;       // the MMA warp's index
-    constexpr int SPW = 128 / NB;              // A: samples of the batch per builder warp (16 or 8)
-    constexpr int RPW = mma_n<D>() / NB;       // B: rows per builder warp
-    constexpr int CPW = 256 / NB;              // accumulator columns per builder warp (3-D)
+    constexpr int NG = mma_groups<D, KAHAN>(); // builder groups: group b builds batches b, b + NG, ...
+    constexpr int NBG = NB / NG;               // warps of a group
+    constexpr int SPW = 128 / NBG;             // A: samples of the batch per builder warp (32 or 8)
+    constexpr int RPW = mma_n<D>() / NBG;      // B: rows per builder warp
+    constexpr int DPW = 256 / NBG;             // accumulator columns per builder warp and drain (3-D)
+    constexpr int CPW = 256 / NB;              // accumulator columns per builder warp at the end (3-D)
     using T = MmaTile<D>;
     constexpr int N = mma_n<D>();
     constexpr uint32_t kBOp = N * 128;  // one B operand: N rows x 128 B
@@ -257,12 +274,14 @@ __global__ void __launch_bounds__(mma_threads<KAHAN>(), KAHAN ? 1 : 2) k_spread_
     extern __shared__ unsigned char smem_mma_raw[];
     unsigned char *sm = smem_mma_raw + ((1024u - (smem_addr(smem_mma_raw) & 1023u)) & 1023u);
     unsigned char *opB = sm;  // [buf][hi, lo][N rows x 128 B], SW128
-    unsigned char *stage = sm + kMmaStageOff;
-    uint64_t *full = reinterpret_cast<uint64_t *>(sm + kMmaBarOff);
-    uint64_t *empty = full + kMmaSlots;
-    uint64_t *ops = empty + kMmaSlots;
-    uint64_t *done = ops + 2;
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(done + 2);
+    using Cfg = MmaCfg<D, KAHAN>;
+    constexpr int BUFS = Cfg::BUFS, SLOTS = Cfg::SLOTS;
+    unsigned char *stage = sm + Cfg::STAGE;
+    uint64_t *full = reinterpret_cast<uint64_t *>(sm + Cfg::BAR);
+    uint64_t *empty = full + SLOTS;
+    uint64_t *ops = empty + SLOTS;
+    uint64_t *done = ops + BUFS;
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(done + BUFS);
 
     const Geom &g = a.g;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -287,12 +306,12 @@ __global__ void __launch_bounds__(mma_threads<KAHAN>(), KAHAN ? 1 : 2) k_spread_
         tmem_relinquish();
     }
     if (threadIdx.x == 0) {
-        for (int k = 0; k < kMmaSlots; ++k) {
+        for (int k = 0; k < SLOTS; ++k) {
             mbar_init(&full[k], 32);                  // the loader warp, every lane
-            mbar_init(&empty[k], NB * 32);  // every builder lane
+            mbar_init(&empty[k], NBG * 32);  // every builder lane of the batch's group
         }
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(&ops[b], NB * 32);
+        for (int b = 0; b < BUFS; ++b) {
+            mbar_init(&ops[b], NBG * 32);
             mbar_init(&done[b], 1);                   // tcgen05.commit
         }
         fence_barrier_init();
@@ -311,9 +330,11 @@ __global__ void __launch_bounds__(mma_threads<KAHAN>(), KAHAN ? 1 : 2) k_spread_
             int o[3], e[3];
             tile_coords<D>(g, sub.x % g.ntiles, o, e);
             const int lw = warp - NB;
+            const bool vec = a.c_coil == 1 && a.c_elem % 2 == 0 && cg0 + CG <= g.n_coil &&
+                             (reinterpret_cast<uintptr_t>(a.c) & 15) == 0;
             const int ns = g.ns;
             for (int k = lw; k < nb; k += kMmaLoaders) {
-                const int slot = k % kMmaSlots;
+                const int slot = k % SLOTS;
                 const int n = min(B, sub.z - k * B);
                 const bool ok = lane < n;
                 float4 pt = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -324,13 +345,27 @@ __global__ void __launch_bounds__(mma_threads<KAHAN>(), KAHAN ? 1 : 2) k_spread_
                 }
                 float sw = 1.f;
                 if (ok && a.weight) sw = a.weight[j];
+                // the 8 coil values of each sample: where they are one aligned 64-byte run, four
+                // lanes read a sample's together (16 bytes each, 8 samples an instruction: a
+                // quarter of the sectors per request of a lane reading its own sample)
+                float4 v4[4];
                 float2 v[CG];
+                if (vec) {
 #pragma unroll
-                for (int cc = 0; cc < CG; ++cc) {
-                    v[cc] = make_float2(0.f, 0.f);
-                    if (ok && cg0 + cc < g.n_coil) {
-                        const float2 tv = a.c[(int64_t)j * a.c_elem + (int64_t)(cg0 + cc) * a.c_coil];
-                        v[cc] = make_float2(tv.x * sw, tv.y * sw);
+                    for (int i = 0; i < 4; ++i) {
+                        const int s8 = 8 * i + (lane >> 2);
+                        const uint32_t js = __shfl_sync(0xffffffffu, j, s8);
+                        v4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (s8 < n)
+                            v4[i] = *reinterpret_cast<const float4 *>(a.c + (int64_t)js * a.c_elem + cg0 +
+                                                                      2 * (lane & 3));
+                    }
+                } else {
+#pragma unroll
+                    for (int cc = 0; cc < CG; ++cc) {
+                        v[cc] = make_float2(0.f, 0.f);
+                        if (ok && cg0 + cc < g.n_coil)
+                            v[cc] = a.c[(int64_t)j * a.c_elem + (int64_t)(cg0 + cc) * a.c_coil];
                     }
                 }
                 int r[3] = {0, 0, 0};
@@ -346,26 +381,43 @@ __global__ void __launch_bounds__(mma_threads<KAHAN>(), KAHAN ? 1 : 2) k_spread_
                     }
                 }
                 // the slot's previous batch must be released by every builder lane
-                if (k >= kMmaSlots &&
-                    !mbar_wait_bounded(&empty[slot], (uint32_t)((k / kMmaSlots - 1) & 1)) && lane == 0)
+                if (k >= SLOTS &&
+                    !mbar_wait_bounded(&empty[slot], (uint32_t)((k / SLOTS - 1) & 1)) && lane == 0)
                     atomicOr(status, kStatusSpreadTimeout);
                 unsigned char *sl = stage + (size_t)slot * kMmaSlotBytes;
-                // per grid dimension: the distance of tile plane 0 from the sample (plane t:
-                // d0 - t) and the plane of the first tap; a lane without a sample gets a first
-                // tap no plane reaches, so all its weights are 0
-                float *d0 = reinterpret_cast<float *>(sl + kMmaStD0);
-                int *rs = reinterpret_cast<int *>(sl + kMmaStR);
-                d0[lane] = pt.x + (float)(ns - 1 + r[0]);
-                d0[B + lane] = pt.y + (float)(ns - 1 + r[1]);
-                rs[lane] = ok ? r[0] : -(1 << 20);
-                rs[B + lane] = ok ? r[1] : -(1 << 20);
-                if constexpr (D == 3) {
-                    d0[2 * B + lane] = pt.z + (float)(ns - 1 + r[2]);
-                    rs[2 * B + lane] = ok ? r[2] : -(1 << 20);
+                // the sample's tile-plane weights (28 in 3-D, 24 in 2-D); a lane without a
+                // sample gets a first tap no plane reaches, so all its weights are 0
+                const float pf[3] = {pt.x, pt.y, pt.z};
+#pragma unroll
+                for (int d = 0; d < D; ++d) {
+                    constexpr int OFF = 3 - D;  // 2-D: the axes are the tile's y and z planes
+                    const int planes = d + OFF == 0 ? kMmaTX : (d + OFF == 1 ? kMmaTY : kMmaTZ);
+                    float *wp = reinterpret_cast<float *>(
+                        sl + (d + OFF == 0 ? kMmaStWx : (d + OFF == 1 ? kMmaStWy : kMmaStWz)));
+                    const float d0 = pf[d] + (float)(ns - 1 + r[d]);
+                    const int rs = ok ? r[d] : -(1 << 20);
+                    const float beta = g.beta2[d];
+#pragma unroll
+                    for (int t = 0; t < planes; ++t) {
+                        const float dd = d0 - (float)t;
+                        const float wv = ex2_approx(-beta * dd * dd);
+                        wp[t * kMmaWS + lane] = (unsigned)(t - rs) < (unsigned)W ? wv : 0.f;
+                    }
                 }
                 float2 *vs = reinterpret_cast<float2 *>(sl + kMmaStV);
+                if (vec) {
 #pragma unroll
-                for (int cc = 0; cc < CG; ++cc) vs[cc * B + lane] = v[cc];
+                    for (int i = 0; i < 4; ++i) {
+                        const int s8 = 8 * i + (lane >> 2);
+                        const float ws = __shfl_sync(0xffffffffu, sw, s8);
+                        float2 *vp = vs + 2 * (lane & 3) * kMmaVS + s8;
+                        vp[0] = make_float2(v4[i].x * ws, v4[i].y * ws);
+                        vp[kMmaVS] = make_float2(v4[i].z * ws, v4[i].w * ws);
+                    }
+                } else {
+#pragma unroll
+                    for (int cc = 0; cc < CG; ++cc) vs[cc * kMmaVS + lane] = make_float2(v[cc].x * sw, v[cc].y * sw);
+                }
                 mbar_arrive(&full[slot]);
             }
         } else if (warp == WM) {
@@ -374,10 +426,10 @@ __global__ void __launch_bounds__(mma_threads<KAHAN>(), KAHAN ? 1 : 2) k_spread_
                 constexpr uint32_t idesc = tc_idesc_tf32(kMmaM, N);
                 const uint32_t b0 = smem_addr(opB);
                 for (int k = 0; k < nb; ++k) {
-                    const int buf = k & 1;
-                    if (!mbar_wait_bounded(&ops[buf], (uint32_t)((k >> 1) & 1))) atomicOr(status, kStatusSpreadTimeout);
+                    const int buf = k % BUFS;
+                    if (!mbar_wait_bounded(&ops[buf], (uint32_t)((k / BUFS) & 1))) atomicOr(status, kStatusSpreadTimeout);
                     tc_fence_after();
-                    const uint32_t ah = tbase + 64u * buf, al = ah + 32u;
+                    const uint32_t ah = tbase + Cfg::a_col(buf), al = ah + 32u;
                     const uint32_t d = tbase + kMmaColD + (KAHAN ? 64u * buf : 0u);
                     // K step jk starts 32 jk bytes further: + 2 jk in the descriptor's address
                     // field (16-byte units; shared addresses stay far below its 14-bit range)
@@ -400,47 +452,24 @@ __global__ void __launch_bounds__(mma_threads<KAHAN>(), KAHAN ? 1 : 2) k_spread_
             // warp (q, hk): TMEM quarter q; A for samples SPW hk .. SPW hk + SPW - 1 of a batch;
             // B rows RPW warp .. (3-D: x plane bx, coils bc0 .. bc0 + RPW / 2 - 1); the
             // accumulator's columns CPW hk .. (3-D)
-            const int q = warp & 3, hk = warp >> 2;
+            const int wg = warp % NBG, grp_b = warp / NBG;
+            const int q = wg & 3, hk = wg >> 2;
             const int m = 32 * q + lane, y = m >> 4, z = m & 15;  // tile cell (y, z) of TMEM lane m
-            const int bx = (RPW * warp) >> 4, bc0 = ((RPW * warp) & 15) >> 1;
             const uint32_t tl = tmem_lane_base(tbase, q);
-            for (int k = 0; k < nb; ++k) {
-                const int slot = k % kMmaSlots, buf = k & 1;
-                if (!mbar_wait_bounded(&full[slot], (uint32_t)((k / kMmaSlots) & 1)) && lane == 0)
+            float *ssum = D == 3 && !KAHAN ? reinterpret_cast<float *>(sm + Cfg::SUM) + m : nullptr;
+            for (int k = grp_b; k < nb; k += NG) {
+                const int slot = k % SLOTS, buf = k % BUFS;
+                if (!mbar_wait_bounded(&full[slot], (uint32_t)((k / SLOTS) & 1)) && lane == 0)
                     atomicOr(status, kStatusSpreadTimeout);
-                {
-                    // the batch's tile-plane weights per sample (28 in 3-D, 24 in 2-D), shared
-                    // by the builder warps: warp b computes planes b, b + 8, ... of sample `lane`
-                    unsigned char *slw = stage + (size_t)slot * kMmaSlotBytes;
-                    const float *d0 = reinterpret_cast<const float *>(slw + kMmaStD0);
-                    const int *rs = reinterpret_cast<const int *>(slw + kMmaStR);
-                    constexpr int XT = D == 3 ? kMmaTX : 0;  // planes along N's grid dimension
-#pragma unroll
-                    for (int i = 0; i < (T::TAPS + NB - 1) / NB; ++i) {
-                        const int jt = warp + NB * i;
-                        if (jt >= T::TAPS) break;
-                        const int reg = jt < XT ? 0 : (jt < XT + kMmaTY ? 1 : 2);  // x, y or z planes
-                        const int t = jt - (reg == 0 ? 0 : (reg == 1 ? XT : XT + kMmaTY));
-                        const int gd = D == 3 ? reg : reg - 1;  // grid dimension (2-D: y, z planes only)
-                        const float d = d0[gd * B + lane] - (float)t;
-                        // (a parameter array indexed at run time would be copied to local memory)
-                        const float beta = gd == 0 ? g.beta2[0] : (gd == 1 ? g.beta2[1] : g.beta2[2]);
-                        const float wv = ex2_approx(-beta * d * d);
-                        const bool in = (unsigned)(t - rs[gd * B + lane]) < (unsigned)W;
-                        reinterpret_cast<float *>(slw + (reg == 0 ? kMmaStWx : (reg == 1 ? kMmaStWy : kMmaStWz)))
-                            [t * kMmaWS + lane] = in ? wv : 0.f;
-                    }
-                    asm volatile("bar.sync 1, %0;" ::"n"(NB * 32) : "memory");
-                }
-                // the MMAs of batch k - 2 (same operand buffer) have completed
-                if (k >= 2 && !mbar_wait_bounded(&done[buf], (uint32_t)(((k >> 1) - 1) & 1)) && lane == 0)
+                // the MMAs of batch k - BUFS (same operand buffer) have completed
+                if (k >= BUFS && !mbar_wait_bounded(&done[buf], (uint32_t)((k / BUFS - 1) & 1)) && lane == 0)
                     atomicOr(status, kStatusSpreadTimeout);
                 if constexpr (KAHAN) {
                     if (k >= 2) {
                         // batch k - 2's accumulator D[k % 2] into the group sum before batch k
                         // overwrites it
                         tc_fence_after();
-                        mma_drain_batch_k2<CPW / 16>(tl, CPW * hk, kMmaColD + 64u * buf, k - 2);
+                        mma_drain_batch_k2<DPW / 16>(tl, DPW * hk, kMmaColD + 64u * buf, k - 2);
                     }
                 }
                 const unsigned char *sl = stage + (size_t)slot * kMmaSlotBytes;
@@ -465,18 +494,19 @@ __global__ void __launch_bounds__(mma_threads<KAHAN>(), KAHAN ? 1 : 2) k_spread_
                         lo[4 * i + 2] = l1.x;
                         lo[4 * i + 3] = l1.y;
                     }
-                    tmem_st_x8(tl + 64u * buf + SPW * hk + 8u * h, hi);
-                    tmem_st_x8(tl + 64u * buf + 32u + SPW * hk + 8u * h, lo);
+                    tmem_st_x8(tl + Cfg::a_col(buf) + SPW * hk + 8u * h, hi);
+                    tmem_st_x8(tl + Cfg::a_col(buf) + 32u + SPW * hk + 8u * h, lo);
                 }
                 const float2 *vs = reinterpret_cast<const float2 *>(sl + kMmaStV);
                 unsigned char *bh = opB + (size_t)(2 * buf) * kBOp, *bl = bh + kBOp;
                 if constexpr (D == 3) {
-                    // B: rows (x = bx, coils bc0 .. bc0 + RPW / 2 - 1, re/im) for sample `lane`
-                    const float wxk = reinterpret_cast<const float *>(sl + kMmaStWx)[bx * kMmaWS + lane];
+                    // B: rows RPW wg .. (x plane, coil, re/im) for sample `lane`
 #pragma unroll
                     for (int cc = 0; cc < RPW / 2; ++cc) {
-                        const float2 vv = vs[(bc0 + cc) * B + lane];
-                        const int nre = bx * 16 + (bc0 + cc) * 2;
+                        const int nre = RPW * wg + 2 * cc;  // row: 16 x + 2 coil
+                        const float wxk =
+                            reinterpret_cast<const float *>(sl + kMmaStWx)[(nre >> 4) * kMmaWS + lane];
+                        const float2 vv = vs[((nre & 15) >> 1) * kMmaVS + lane];
                         float2 h, l;
                         tf32_split2(make_float2(wxk, wxk), vv, h, l);
                         *reinterpret_cast<float *>(bh + sw128_offset(nre, lane)) = h.x;
@@ -486,7 +516,7 @@ __global__ void __launch_bounds__(mma_threads<KAHAN>(), KAHAN ? 1 : 2) k_spread_
                     }
                 } else {
                     // B: rows (coil = warp, re/im) for sample `lane`: the coil value itself
-                    const float2 vv = vs[warp * B + lane];
+                    const float2 vv = vs[warp * kMmaVS + lane];
                     float2 h, l;
                     tf32_split2(make_float2(1.f, 1.f), vv, h, l);
                     *reinterpret_cast<float *>(bh + sw128_offset(2 * warp, lane)) = h.x;
@@ -497,12 +527,12 @@ __global__ void __launch_bounds__(mma_threads<KAHAN>(), KAHAN ? 1 : 2) k_spread_
                 mbar_arrive(&empty[slot]);
                 if (!KAHAN && k % kMmaGroup == 0 && k > 0) {
                     // batch k starts a new group: once the previous group's MMAs are done,
-                    // add its accumulator into S (the same phase is waited for again at
-                    // k + 1, which returns at once)
-                    if (!mbar_wait_bounded(&done[(k - 1) & 1], (uint32_t)(((k - 1) >> 1) & 1)) && lane == 0)
+                    // add its accumulator into S.  (The MMAs complete in order and batch k -
+                    // BUFS was waited for above, so this barrier is in batch k - 1's phase.)
+                    if (!mbar_wait_bounded(&done[(k - 1) % BUFS], (uint32_t)(((k - 1) / BUFS) & 1)) && lane == 0)
                         atomicOr(status, kStatusSpreadTimeout);
                     tc_fence_after();
-                    mma_drain<N>(tl, hk, k == kMmaGroup);
+                    mma_drain<N, DPW>(tl, hk, k == kMmaGroup, ssum);
                 }
                 // operands visible to the tensor core before the MMA warp proceeds
                 tmem_wait_st();
@@ -514,20 +544,32 @@ __global__ void __launch_bounds__(mma_threads<KAHAN>(), KAHAN ? 1 : 2) k_spread_
             // ---------------------------------------------------------------- epilogue
             if (nb > 0) {
                 const int kl = nb - 1;
-                if (!mbar_wait_bounded(&done[kl & 1], (uint32_t)((kl >> 1) & 1)) && lane == 0)
+                // (two groups: the group's own last batch first, after which the other buffer's
+                // barrier is in the phase of the block's last batch, so that its parity means
+                // that phase and not the one before)
+                const int ko = NG == 2 ? ((kl & 1) == grp_b ? kl : kl - 1) : kl;
+                if (ko >= 0 && !mbar_wait_bounded(&done[ko % BUFS], (uint32_t)((ko / BUFS) & 1)) && lane == 0)
                     atomicOr(status, kStatusSpreadTimeout);
+                if (NG == 2 && ko != kl && !mbar_wait_bounded(&done[kl % BUFS], (uint32_t)((kl / BUFS) & 1)) && lane == 0)
+                    atomicOr(status, kStatusSpreadTimeout);
+                if constexpr (NG == 2) {
+                    // S, drained by group 0, is read by all builders below
+                    asm volatile("bar.sync 1, %0;" ::"n"(NB * 32) : "memory");
+                }
                 tc_fence_after();
                 if constexpr (KAHAN) {
                     // the last two batches' accumulators, in order
                     for (int j = max(0, nb - 2); j < nb; ++j) {
-                        mma_drain_batch_k2<CPW / 16>(tl, CPW * hk, kMmaColD + 64u * (j & 1), j);
+                        mma_drain_batch_k2<DPW / 16>(tl, DPW * hk, kMmaColD + 64u * (j & 1), j);
                         tmem_wait_st();  // G (and S, C) stored before the next drain reads them
                     }
                     // the last group's sum into S, C (S = G when there was one group)
-                    mma_drain_kahan<CPW / 16>(tl, CPW * hk, kMmaColGK, nb <= kMmaGroup);
+                    mma_drain_kahan<DPW / 16>(tl, DPW * hk, kMmaColGK, nb <= kMmaGroup);
                     tmem_wait_st();
                 }
             }
+            // the tile's columns over all builder warps
+            const int he = warp >> 2;
             // the unit's tile, read again here rather than kept in registers through the loop
             const int4 su = a.subs[unit / n_cg];
             int o[3], e[3];
@@ -536,35 +578,31 @@ __global__ void __launch_bounds__(mma_threads<KAHAN>(), KAHAN ? 1 : 2) k_spread_
             const bool split = (su.w & kSplitFlag) != 0;
             const bool inside = y < e[T::DY] && z < e[T::DZ];
             if constexpr (D == 3) {
-                // this warp: lanes of quarter q, columns CPW hk .. (x planes CPW hk / 16 ..)
+                // this warp: lanes of quarter q, columns CPW he .. (x planes CPW he / 16 ..)
                 const int64_t cell_yz = (int64_t)(o[1] + y) * g.nf[2] + (o[2] + z);
 #pragma unroll
                 for (int xi = 0; xi < CPW / 16; ++xi) {
-                    // columns CPW hk + 16 xi ..: cell x = (CPW / 16) hk + xi, (coil, re/im) pairs
+                    // columns CPW he + 16 xi ..: cell x = (CPW / 16) he + xi, (coil, re/im) pairs
                     float dv[16];
                     if (nb > 0 && KAHAN) {
                         float cv[16];
-                        tmem_ld_x16(tl + kMmaColSK + CPW * hk + 16u * xi, dv);
-                        tmem_ld_x16(tl + kMmaColCK + CPW * hk + 16u * xi, cv);
+                        tmem_ld_x16(tl + kMmaColSK + CPW * he + 16u * xi, dv);
+                        tmem_ld_x16(tl + kMmaColCK + CPW * he + 16u * xi, cv);
                         tmem_wait_ld();
 #pragma unroll
                         for (int i = 0; i < 16; ++i) dv[i] -= cv[i];
                     } else if (nb > 0) {
-                        tmem_ld_x16(tl + kMmaColD + CPW * hk + 16u * xi, dv);
+                        tmem_ld_x16(tl + kMmaColD + CPW * he + 16u * xi, dv);
+                        tmem_wait_ld();
                         if (nb > kMmaGroup) {  // plus the drained groups
-                            float sv[16];
-                            tmem_ld_x16(tl + kMmaColD + N + CPW * hk + 16u * xi, sv);
-                            tmem_wait_ld();
 #pragma unroll
-                            for (int i = 0; i < 16; ++i) dv[i] += sv[i];
-                        } else {
-                            tmem_wait_ld();
+                            for (int i = 0; i < 16; ++i) dv[i] += ssum[(CPW * he + 16 * xi + i) * kMmaM];
                         }
                     } else {
 #pragma unroll
                         for (int i = 0; i < 16; ++i) dv[i] = 0.f;
                     }
-                    const int x = (CPW / 16) * hk + xi;
+                    const int x = (CPW / 16) * he + xi;
                     if (!inside || x >= e[0]) continue;
                     const int64_t cell = (int64_t)(o[0] + x) * g.nf[1] * g.nf[2] + cell_yz;
 #pragma unroll
@@ -580,13 +618,13 @@ __global__ void __launch_bounds__(mma_threads<KAHAN>(), KAHAN ? 1 : 2) k_spread_
                     }
                 }
             } else {
-                // this warp: lanes of quarter q, columns 8 hk .. 8 hk + 7 (coils 4 hk .. 4 hk + 3)
+                // this warp: lanes of quarter q, columns 8 he .. 8 he + 7 (coils 4 he .. 4 he + 3)
                 float dv[8];
                 if (nb > 0) {
-                    tmem_ld_x8(tl + kMmaColD + 8u * hk, dv);
+                    tmem_ld_x8(tl + kMmaColD + 8u * he, dv);
                     if (nb > kMmaGroup) {  // plus the drained groups
                         float sv[8];
-                        tmem_ld_x8(tl + kMmaColD + N + 8u * hk, sv);
+                        tmem_ld_x8(tl + kMmaColD + N + 8u * he, sv);
                         tmem_wait_ld();
 #pragma unroll
                         for (int i = 0; i < 8; ++i) dv[i] += sv[i];
@@ -601,7 +639,7 @@ __global__ void __launch_bounds__(mma_threads<KAHAN>(), KAHAN ? 1 : 2) k_spread_
                     const int64_t cell = (int64_t)(o[0] + y) * g.nf[1] + (o[1] + z);
 #pragma unroll
                     for (int cc = 0; cc < 4; ++cc) {
-                        const int c = 4 * hk + cc;
+                        const int c = 4 * he + cc;
                         if (cg0 + c >= g.n_coil) break;
                         float2 *dst = a.grid + ((int64_t)grp * g.n_coil + cg0 + c) * g.G + cell;
                         if (split) {
