@@ -993,6 +993,20 @@ int plan_create_impl(const gbn_plan_desc *desc, gbn_plan **out) {
             reg_spread = false;
         }
     }
+    // 2-D with wide stencils, unless the caller chose a tile: 32 x 32 tiles in registers
+    if (p->dim == 2 && !tile_given && 2 * p->ns > 16) {
+        Geom w{};
+        w.dim = 2;
+        w.W = 2 * p->ns;
+        for (int d = 0; d < 2; ++d) {
+            w.nf[d] = p->nf[d];
+            w.tile[d] = 32;
+        }
+        if (spread_wide_applies(w)) {
+            ts[0] = ts[1] = 32;
+            reg_spread = false;
+        }
+    }
     // the cube and tensor-core kernels keep a ring of batches full: long work items (the 3-D
     // tensor-core spread and interp share the work items; measured on the 3-D radial
     // workload: interp 3.75 ms at 4096 samples against 3.93 at 2048, spread even)
@@ -1003,6 +1017,8 @@ int plan_create_impl(const gbn_plan_desc *desc, gbn_plan **out) {
     if (few_spread && desc->max_subproblem <= 0) p->interp_max_sub = 256;
     make_geom(p, ts, p->gs);
     make_geom(p, ti, p->gi);
+    // a warp takes ~1 us a sample there: short items keep the dense centre's tail short
+    if (interp_wide_applies(p->gi) && desc->max_subproblem <= 0) p->interp_max_sub = 64;
 
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);

@@ -208,6 +208,11 @@ int spread_path_kind(const Geom &g, int coil_group, int variant, int threads);
 constexpr int kFewMaxCoils = 3;
 bool few_applies(const Geom &g);
 void few_tile(int n_coil, int tile[3]);
+// the wide-stencil 2-D kernels (spread2d_wide.cuh on 32 x 32 tiles, interp2d_wide.cuh) take this
+// geometry
+constexpr int kWideMinW = 18, kWideMaxW = 30;  // taps per axis
+bool spread_wide_applies(const Geom &g);
+bool interp_wide_applies(const Geom &g);
 // kernels launch_spread runs for these arguments (the 3-D register path adds a Kahan instance)
 int spread_kernel_count(const SpreadArgs &a, int64_t n_sub, int coil_group, int threads);
 cudaError_t launch_interp(const InterpArgs &a, int64_t n_sub, int coil_group, int threads,

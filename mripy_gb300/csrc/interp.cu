@@ -5,7 +5,7 @@
 // subproblem, windows gathered by the threads).  3-D with at most 16 taps:
 // k_interp3d_one (one coil per block: plans of 1 to 3 coils), k_interp3d_planes (4 or 8 coils
 // per block, window streamed by x planes) or k_interp3d.
-// Otherwise (1-D, wide stencils): k_interp (one thread per sample).
+// 2-D with 18 to 30 taps: k_interp2d_wide.  Otherwise (1-D, wider stencils): k_interp (one thread per sample).
 #include <algorithm>
 #include <cstring>
 
@@ -13,6 +13,7 @@
 #include "grid2d_kernels.cuh"
 #include "grid3d_kernels.cuh"
 #include "interp2d_tma.cuh"
+#include "interp2d_wide.cuh"
 #include "interp3d_mma.cuh"
 #include "interp3d_one.cuh"
 
@@ -30,12 +31,19 @@ bool interp3d_one_applies(const Geom &g) {
     return b > 0 && b <= 112 * 1024;
 }
 
+// wide 2-D stencils: one coil per block, while the window fits two blocks per SM
+bool interp_wide_applies(const Geom &g) {
+    const size_t b = interp2d_wide_smem(g);
+    return b > 0 && b <= 112 * 1024;
+}
+
 // shared memory of the kernel launch_interp runs for this geometry, coil group and thread
 // count (the 3-D kernel depends on all three)
 size_t interp_smem_bytes(const Geom &g, int coil_group, int threads) {
     if (use_2d_path(g)) return interp2d_smem_bytes(g, coil_group);
     if (const size_t ps = interp3d_planes_smem_bytes(g, coil_group, threads > 256 ? 256 : threads)) return ps;
     if (coil_group == 1 && interp3d_one_applies(g)) return interp3d_one_smem_bytes(g);
+    if (interp_wide_applies(g)) return interp2d_wide_smem(g);
     size_t cells = 1;
     for (int d = 0; d < g.dim; ++d) cells *= (size_t)(g.tile[d] + g.W - 1);
     return cells * (size_t)coil_group * sizeof(float2);
@@ -93,6 +101,13 @@ cudaError_t launch_interp(const InterpArgs &a, int64_t n_sub, int coil_group, in
             }
         }));
         return err;
+    }
+    if (interp_wide_applies(a.g)) {
+        const int vec = (uintptr_t)a.grid % 16 == 0 && a.g.nf[1] % 2 == 0 && a.g.G % 2 == 0;
+        err = set_smem(k_interp2d_wide, smem);
+        if (err != cudaSuccess) return err;
+        k_interp2d_wide<<<dim3((unsigned)n_sub, (unsigned)a.g.n_coil), threads > 256 ? 256 : threads, smem, s>>>(a, vec);
+        return cudaGetLastError();
     }
     if (a.g.dim == 3 && a.g.W <= 16) {
         const int th = threads > 256 ? 256 : threads;

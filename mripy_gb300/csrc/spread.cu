@@ -3,13 +3,15 @@
 // 2-D / 3-D with at most 16 taps per dimension and 4 or 8 coils per block, on the tile shape
 // they are built for: k_spread2d_reg / k_spread3d_reg (accumulators in registers).
 // Other 2-D / 3-D tiles: k_spread2d / k_spread3d (warp-owned shared-memory rows, no atomics).
-// Otherwise (1-D, wide stencils, small grids): k_spread (shared-memory atomics).
-// 3-D with 8 coils per block also: k_spread_mma<3, ...> (tensor cores, 4 x 8 x 16 tiles) and
+// 2-D with 18 to 30 taps: k_spread2d_wide.  Otherwise (1-D, wider stencils, 3-D above 16 taps,
+// small grids): k_spread (shared-memory atomics).
+// 3-D with 1 to 3 coils: k_spread3d_few.  3-D with 8 coils per block also: k_spread_mma<3, ...> (tensor cores, 4 x 8 x 16 tiles) and
 // k_spread3d_cube (register cubes), each followed by the compensated cube instance for the
 // dense work items.
 #include "dispatch.cuh"
 #include "grid2d_kernels.cuh"
 #include "grid3d_kernels.cuh"
+#include "spread2d_wide.cuh"
 #include "spread3d_cube.cuh"
 #include "spread3d_few.cuh"
 #include "spread3d_mma.cuh"
@@ -24,6 +26,7 @@ static bool use_2d_path(const Geom &g) {
 }
 
 size_t spread_smem_bytes(const Geom &g, int coil_group) {
+    if (spread_wide_applies(g)) return kWideSmem;
     if (use_2d_path(g)) return spread2d_smem_bytes(g, coil_group);
     if (grid3d_applies(g)) return spread3d_smem_bytes(g, coil_group);
     size_t cells = 1;
@@ -77,6 +80,12 @@ bool few_applies(const Geom &g) {
 void few_tile(int n_coil, int tile[3]) {
     tile[0] = tile[1] = kFewTile;
     tile[2] = few_tz(n_coil);
+}
+
+// the wide-stencil 2-D spread applies: its tile, a grid of at least tile + stencil cells per axis
+bool spread_wide_applies(const Geom &g) {
+    return g.dim == 2 && g.W >= kWideMinW && g.W <= kWideMaxW && g.tile[0] == kWideTile && g.tile[1] == kWideTile &&
+           g.nf[0] >= kWideTile + g.W && g.nf[1] >= kWideTile + g.W;
 }
 
 // the cube and tensor-core kernels read interleaved work items
@@ -168,6 +177,10 @@ cudaError_t launch_spread(const SpreadArgs &a, int64_t n_sub, int coil_group, in
     if (mma_path(a.g, coil_group, a.variant)) {
         GBN_DISPATCH_W(a.g.W, { err = launch_mma<WT>(a, n_sub, s); });
         return err;
+    }
+    if (spread_wide_applies(a.g)) {
+        k_spread2d_wide<<<dim3((unsigned)n_sub, (unsigned)a.g.n_coil), kWideWarps * 32, kWideSmem, s>>>(a);
+        return cudaGetLastError();
     }
     // few-coil 3-D kernel
     if (few_applies(a.g)) {
