@@ -89,6 +89,7 @@ struct gbn_plan {
     bool spread_items_interleaved = false;  // split tiles' work items interleave (cube kernel)
     int dense_min = kDenseDefault;  // 3-D spread tiles with this many samples use compensated sums (0: never)
     int64_t n_dense_sub = 0;
+    bool rows_sorted = false;  // a tile's entries of the spread list are in the order of their y rows
     int64_t n_split = 0;  // spread tiles covered by more than one subproblem (listed in split_tiles)
     int64_t G = 1, n_inst = 1;
     size_t device_bytes = 0;
@@ -498,7 +499,8 @@ bool grid_tensor_map3d(gbn_plan *p, const float2 *grid, int cg, int BY, int BZ) 
 
 // the tensor-core interp runs this plan's interps (on the spread's tiles and work lists)
 bool interp_on_tensor_cores(const gbn_plan *p) {
-    return p->interp_variant != 1 && interp_mma_applies(p->gs, spread_cg(p));
+    return p->interp_variant != 1 && interp_mma_applies(p->gs, spread_cg(p)) &&
+           (p->rows_sorted || !p->points_set);
 }
 
 int run_interp(gbn_plan *p, const float2 *grid, void *c, gbn_layout L, const float *weight, cudaStream_t s) {
@@ -508,6 +510,7 @@ int run_interp(gbn_plan *p, const float2 *grid, void *c, gbn_layout L, const flo
         m.g = p->gs;
         m.subs = p->spread_subs.as<int4>();
         m.idx = p->dup_idx.as<uint32_t>();
+        m.keys = p->dup_keys_sorted.as<uint32_t>();
         m.pts_by_sample = p->pts.as<float4>();
         m.grid = grid;
         m.c = (float2 *)c;
@@ -685,9 +688,13 @@ int set_points_impl(gbn_plan *p, int dtype, const void *x, const void *y, const 
         bound *= std::min<uint64_t>(per, (uint64_t)g.ntile[d]);
     }
     const bool early = M > 0 && bound <= kOneSyncEntries;
+    // the 3-D tensor-core kernels skip the y rows that none of a batch's samples reaches: a
+    // tile's entries are sorted by their stencil's first row (one more radix pass of the sort)
+    const bool y_class = interp_mma_applies(p->gs, spread_cg(p)) && Ts < ((int64_t)1 << (32 - kYClassBits));
+    p->rows_sorted = y_class;
     auto dup_keys = [&]() -> int {
         GBN_CUDA(launch_dup_keys(p->pts.as<float4>(), M, p->traj_off_d.as<int64_t>(), p->gs, to,
-                                 p->dup_keys.as<uint32_t>(), p->dup_vals.as<uint32_t>(), s));
+                                 p->dup_keys.as<uint32_t>(), p->dup_vals.as<uint32_t>(), y_class, s));
         return GBN_OK;
     };
     if (early) {
@@ -726,7 +733,7 @@ int set_points_impl(gbn_plan *p, int dtype, const void *x, const void *y, const 
     if (E > 0) {
         uint32_t *kin = p->dup_keys.as<uint32_t>(), *vin = p->dup_vals.as<uint32_t>();
         uint32_t *kout = p->dup_keys_sorted.as<uint32_t>(), *vout = p->dup_idx.as<uint32_t>();
-        const int bits = key_bits((uint64_t)Ts);
+        const int bits = key_bits((uint64_t)Ts) + (y_class ? kYClassBits : 0);
         GBN_TRY(cub_call(p, [&](void *tmp, size_t &bytes) {
             return cub::DeviceRadixSort::SortPairs(tmp, bytes, kin, kout, vin, vout, (int)E, 0, bits, s);
         }));

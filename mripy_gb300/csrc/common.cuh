@@ -114,7 +114,8 @@ struct PrepArgs {
 };
 cudaError_t launch_prep(int coord_dtype, PrepArgs a, cudaStream_t s);
 cudaError_t launch_dup_keys(const float4 *pts, int64_t M, const int64_t *d_traj_off, const Geom &gs,
-                            const uint64_t *touch_off, uint32_t *keys, uint32_t *vals, cudaStream_t s);
+                            const uint64_t *touch_off, uint32_t *keys, uint32_t *vals, bool y_class, cudaStream_t s);
+constexpr int kYClassBits = 5;  // W + tile rows - 1 <= 16 + 8 - 1 classes
 // out[i] = pts[idx[i]] for both lists
 cudaError_t launch_gather_pts(const float4 *pts, const uint32_t *idx, int64_t n, float4 *out, const uint32_t *idx2,
                               int64_t n2, float4 *out2, cudaStream_t s);
@@ -185,6 +186,7 @@ struct MmaInterpArgs {
     Geom g;                       // the spread's geometry (4 x 8 x 16 tiles)
     const int4 *subs;             // the spread's work items
     const uint32_t *idx;          // (sample, tile) list: sample index per entry
+    const uint32_t *keys;         // and its sorted key, whose low kYClassBits order a tile's rows
     const float4 *pts_by_sample;  // per sample: in-cell fractions, first-tap cells
     const float2 *grid;
     float2 *c;                    // output samples (zeroed by the launcher)

@@ -18,13 +18,21 @@
 // batch of 128 of the unit's samples:
 // * 8 builder warps: warp (q, h) takes samples 32 q .. 32 q + 31 of the batch, one per lane
 //   (TMEM lane = sample), reads its record, computes its plane weights (ex2.approx) and writes
-//   A in four chunks of 32 columns (y rows 2 c and 2 c + 1; warp h writes row 2 c + h) into
-//   two TMEM chunk buffers, hi and lo parts, arriving on the buffer's `ops` mbarrier; after
-//   the batch it finishes the previous batch: reads its 32 columns of T (coils 4 h .. 4 h + 3,
-//   every x) from TMEM, contracts them with wx and adds them to the output.
+//   A in chunks of 32 columns (two y rows), hi and lo parts; group h (4 warps) builds every
+//   other chunk into its own TMEM buffer and arrives on the buffer's `ops` mbarrier; after
+//   the batch a warp finishes the previous batch: reads its 32 columns of T (coils 4 h .. 4 h +
+//   3, every x) from TMEM, contracts them with wx and adds them to the output.
 // * 1 MMA warp: allocates 256 TMEM columns (A chunks 0..127, two accumulators T 128..255) and
 //   issues per chunk 4 K steps x 3 MMAs (hi * hi, hi * lo, lo * hi) into the batch's T,
 //   committing each chunk to its buffer's `done` mbarrier and the batch to `tfull`.
+// A tile's entries are sorted by the first y row of their stencils, so a batch's samples reach
+// a run of chunks (2.7 of the 4 on average at 12 taps) and the others are skipped.
+//
+// What bounds it: the tensor pipe and the builders together; either alone leaves 2.0 to 2.2 of
+// the 3.1 ms, since a group's chunk waits for the MMAs of the one before.  2.56 M samples x 8
+// coils on 256^3, 12 taps: 3.13 ms with all warps on every chunk, 3.10 with two groups, 2.83
+// with the unreached chunks skipped (12 coils, 576,000 samples: 1.43, 1.31, 1.21).  Chunks of
+// one row in four buffers took 3.51: a chunk's handshake costs more than the overlap gains.
 // Every wait is bounded (kTmaWaitLimit probes); one that gives up sets kStatusSpreadTimeout
 // in the plan's status word and goes on.
 #pragma once
@@ -54,6 +62,17 @@ static_assert(kImSmemBytes > 228 * 1024 / 3, "two blocks per SM at most");
 // byte offset of B element (row n, K index k = y * 16 + z): K atom k / 32, 128-byte swizzle
 __device__ __forceinline__ uint32_t im_b_offset(int n, int k) {
     return (uint32_t)(k >> 5) * kImBAtom + sw128_offset(n, k & 31);
+}
+
+// The chunks (pairs of y rows) that a batch's samples reach: c0 .. c1.  The unit's entries are in
+// the order of their stencils' first rows, which the keys' low bits hold.
+struct ImRows {
+    int c0, c1;
+};
+__device__ __forceinline__ ImRows im_rows(uint32_t first, uint32_t last, int W) {
+    const int lo = (int)(first & ((1u << kYClassBits) - 1)) - (W - 1);
+    const int hi = (int)(last & ((1u << kYClassBits) - 1));  // last row: first row + W - 1
+    return ImRows{max(lo, 0) >> 1, min(hi, kMmaTY - 1) >> 1};
 }
 
 template <int WT>
@@ -88,7 +107,7 @@ __global__ void __launch_bounds__(kImThreads, 2) k_interp3d_mma(MmaInterpArgs a,
     }
     if (threadIdx.x == 0) {
         for (int b = 0; b < 2; ++b) {
-            mbar_init(&ops[b], kImBuilders * 32);
+            mbar_init(&ops[b], kImBuilders / 2 * 32);  // the chunk's group
             mbar_init(&done[b], 1);
             mbar_init(&tfull[b], 1);
             mbar_init(&tempty[b], kImBuilders * 32);
@@ -169,6 +188,11 @@ __global__ void __launch_bounds__(kImThreads, 2) k_interp3d_mma(MmaInterpArgs a,
     __syncthreads();
     tc_fence_after();
     const uint32_t tbase = *tslot;
+    // the sorted key of batch b's first or last entry
+    auto row_key = [&](int b, bool last) {
+        const int i = last ? min(sub.z, (b + 1) * B) - 1 : b * B;
+        return a.keys[(int64_t)sub.y + (int64_t)i * stride];
+    };
 
     if (warp == kImWarp) {
         // ---------------------------------------------------------------- MMA warp
@@ -177,22 +201,28 @@ __global__ void __launch_bounds__(kImThreads, 2) k_interp3d_mma(MmaInterpArgs a,
             // descriptors of B's first K step; a K step's offset adds (bytes / 16) to the
             // address field (shared addresses stay far below its 14-bit range)
             const uint64_t dbh = tc_desc_sw128(smem_addr(bh)), dbl = tc_desc_sw128(smem_addr(bl));
+            int cnt = 0;  // chunks so far: chunk cnt is in buffer cnt & 1
+            uint32_t kf = row_key(0, false), kl = row_key(0, true);
             for (int b = 0; b < nb; ++b) {
                 const int tb = b & 1;
+                const ImRows rows = im_rows(kf, kl, W);
+                if (b + 1 < nb) {
+                    kf = row_key(b + 1, false);
+                    kl = row_key(b + 1, true);
+                }
                 // T[tb] was read out by the builders (batch b - 2)
                 if (b >= 2 && !mbar_wait_bounded(&tempty[tb], (uint32_t)(((b >> 1) - 1) & 1)))
                     atomicOr(status, kStatusSpreadTimeout);
                 const uint32_t d = tbase + kImColT + 64u * tb;
-#pragma unroll
-                for (int ch = 0; ch < 4; ++ch) {
-                    const int gch = 4 * b + ch, buf = gch & 1;
-                    if (!mbar_wait_bounded(&ops[buf], (uint32_t)((gch >> 1) & 1))) atomicOr(status, kStatusSpreadTimeout);
+                for (int ch = rows.c0; ch <= rows.c1; ++ch, ++cnt) {
+                    const int buf = cnt & 1;
+                    if (!mbar_wait_bounded(&ops[buf], (uint32_t)((cnt >> 1) & 1))) atomicOr(status, kStatusSpreadTimeout);
                     tc_fence_after();
                     const uint32_t ah = tbase + 64u * buf, al = ah + 32u;
 #pragma unroll
                     for (int ks = 0; ks < 4; ++ks) {
                         const uint64_t kb = ((uint64_t)ch * kImBAtom + 32u * ks) >> 4;
-                        tc_mma_tf32_ts(d, ah + 8u * ks, dbh + kb, idesc, (ch | ks) != 0);
+                        tc_mma_tf32_ts(d, ah + 8u * ks, dbh + kb, idesc, (ch != rows.c0 || ks != 0) ? 1u : 0u);
                         tc_mma_tf32_ts(d, ah + 8u * ks, dbl + kb, idesc, 1u);
                         tc_mma_tf32_ts(d, al + 8u * ks, dbh + kb, idesc, 1u);
                     }
@@ -215,6 +245,8 @@ __global__ void __launch_bounds__(kImThreads, 2) k_interp3d_mma(MmaInterpArgs a,
         // sample record half way through, so neither load is waited for where it is used
         float4 ptn = make_float4(0.f, 0.f, 0.f, 0.f);
         if (okn) ptn = a.pts_by_sample[jn];
+        int cnt = 0;  // chunks so far: chunk cnt is in buffer cnt & 1, built by group cnt & 1
+        uint32_t kf = row_key(0, false), kl = row_key(0, true);
         for (int b = 0; b <= nb; ++b) {
             float wx[4] = {0.f, 0.f, 0.f, 0.f};
             uint32_t j = 0;
@@ -257,33 +289,43 @@ __global__ void __launch_bounds__(kImThreads, 2) k_interp3d_mma(MmaInterpArgs a,
                     const float wv = ex2_approx(-g.beta2[2] * d * d);
                     wz[t] = (unsigned)(t - r[2]) < (unsigned)W ? wv : 0.f;
                 }
-#pragma unroll
-                for (int ch = 0; ch < 4; ++ch) {
-                    const int gch = 4 * b + ch, buf = gch & 1;
-                    // the MMAs of chunk gch - 2 (same buffer) have completed
-                    if (gch >= 2 && !mbar_wait_bounded(&done[buf], (uint32_t)(((gch >> 1) - 1) & 1)) && lane == 0)
+                if (okn) ptn = a.pts_by_sample[jn];
+                const ImRows rows = im_rows(kf, kl, W);
+                if (b + 1 < nb) {
+                    kf = row_key(b + 1, false);
+                    kl = row_key(b + 1, true);
+                }
+                // this group's chunks: every other one, in its own buffer h
+#pragma unroll 1
+                for (int ch = rows.c0 + ((cnt ^ h) & 1); ch <= rows.c1; ch += 2) {
+                    const int c = cnt + ch - rows.c0;
+                    // the MMAs of chunk c - 2 (same buffer) have completed
+                    if (c >= 2 && !mbar_wait_bounded(&done[h], (uint32_t)(((c >> 1) - 1) & 1)) && lane == 0)
                         atomicOr(status, kStatusSpreadTimeout);
-                    if (ch == 1 && okn) ptn = a.pts_by_sample[jn];
-                    const int y = 2 * ch + h;
-                    const float dy = d0y - (float)y;
-                    const float wyv = ex2_approx(-g.beta2[1] * dy * dy);
-                    const float wy = (unsigned)(y - r[1]) < (unsigned)W ? wyv : 0.f;
-                    float hi[16], lo[16];
 #pragma unroll
-                    for (int t = 0; t < kMmaTZ; t += 2) {
-                        float2 hh, ll;
-                        tf32_split2(make_float2(wy, wy), make_float2(wz[t], wz[t + 1]), hh, ll);
-                        hi[t] = hh.x;
-                        hi[t + 1] = hh.y;
-                        lo[t] = ll.x;
-                        lo[t + 1] = ll.y;
+                    for (int yr = 0; yr < 2; ++yr) {
+                        const int y = 2 * ch + yr;
+                        const float dy = d0y - (float)y;
+                        const float wyv = ex2_approx(-g.beta2[1] * dy * dy);
+                        const float wy = (unsigned)(y - r[1]) < (unsigned)W ? wyv : 0.f;
+                        float hi[16], lo[16];
+#pragma unroll
+                        for (int t = 0; t < kMmaTZ; t += 2) {
+                            float2 hh, ll;
+                            tf32_split2(make_float2(wy, wy), make_float2(wz[t], wz[t + 1]), hh, ll);
+                            hi[t] = hh.x;
+                            hi[t + 1] = hh.y;
+                            lo[t] = ll.x;
+                            lo[t + 1] = ll.y;
+                        }
+                        tmem_st_x16(tl + 64u * h + 16u * yr, hi);
+                        tmem_st_x16(tl + 64u * h + 32u + 16u * yr, lo);
                     }
-                    tmem_st_x16(tl + 64u * buf + 16u * h, hi);
-                    tmem_st_x16(tl + 64u * buf + 32u + 16u * h, lo);
                     tmem_wait_st();
                     tc_fence_before();
-                    mbar_arrive(&ops[buf]);
+                    mbar_arrive(&ops[h]);
                 }
+                cnt += rows.c1 - rows.c0 + 1;
             }
             if (b >= 1) {
                 // epilogue of batch b - 1: coils 4 h .. 4 h + 3, every x plane

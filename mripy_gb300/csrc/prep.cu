@@ -127,10 +127,12 @@ __global__ void __launch_bounds__(256) k_prep(PrepArgs a) {
     }
 }
 
-// the (sample, tile) entries, each sample's adjacent
+// The (sample, tile) entries, each sample's adjacent.  y_class: the key's low kYClassBits hold
+// the stencil's first y row in the tile (+ W - 1: 0 is a stencil that reaches row 0 only), so
+// that the sort leaves a tile's samples in the order of the rows they reach.
 __global__ void k_dup_keys(const float4 *__restrict__ pts, int64_t M, const int64_t *__restrict__ traj_off,
                            Geom gs, const uint64_t *__restrict__ touch_off, uint32_t *__restrict__ keys,
-                           uint32_t *__restrict__ vals) {
+                           uint32_t *__restrict__ vals, int y_class) {
     int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (j >= M) return;
     const int dim = gs.dim;
@@ -149,9 +151,13 @@ __global__ void k_dup_keys(const float4 *__restrict__ pts, int64_t M, const int6
         int ta = (t0[0] + a) % gs.ntile[0];
         for (int b = 0; b < n[1]; ++b) {
             int tb = (t0[1] + b) % gs.ntile[1];
+            int r = c0[1] - tb * gs.tile[1];  // signed first row, as the kernels take it
+            r += r < 0 ? gs.nf[1] : 0;
+            r -= r > gs.nf[1] - gs.W ? gs.nf[1] : 0;
             for (int q = 0; q < n[2]; ++q) {
                 int tq = (t0[2] + q) % gs.ntile[2];
-                keys[pos] = base + (uint32_t)((ta * gs.ntile[1] + tb) * gs.ntile[2] + tq);
+                const uint32_t key = base + (uint32_t)((ta * gs.ntile[1] + tb) * gs.ntile[2] + tq);
+                keys[pos] = y_class ? key << kYClassBits | (uint32_t)(r + gs.W - 1) : key;
                 vals[pos] = (uint32_t)j;
                 ++pos;
             }
@@ -300,9 +306,9 @@ cudaError_t launch_prep(int coord_dtype, PrepArgs a, cudaStream_t s) {
 }
 
 cudaError_t launch_dup_keys(const float4 *pts, int64_t M, const int64_t *d_traj_off, const Geom &gs,
-                            const uint64_t *touch_off, uint32_t *keys, uint32_t *vals, cudaStream_t s) {
+                            const uint64_t *touch_off, uint32_t *keys, uint32_t *vals, bool y_class, cudaStream_t s) {
     if (M == 0) return cudaSuccess;
-    k_dup_keys<<<blocks_for(M, 256), 256, 0, s>>>(pts, M, d_traj_off, gs, touch_off, keys, vals);
+    k_dup_keys<<<blocks_for(M, 256), 256, 0, s>>>(pts, M, d_traj_off, gs, touch_off, keys, vals, y_class ? 1 : 0);
     return cudaGetLastError();
 }
 

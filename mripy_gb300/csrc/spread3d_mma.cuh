@@ -95,7 +95,8 @@ constexpr uint32_t kMmaStWz = kMmaStWy + 4 * kMmaTY * kMmaWS;           // [TZ][
 constexpr int kMmaVS = kMmaBatch + 2;  // float2 per staged coil row: the four 16-byte quarters of a
                                        // sample's coils are stored to distinct banks
 constexpr uint32_t kMmaStV = kMmaStWz + 4 * kMmaTZ * kMmaWS;            // [8 coils][kMmaVS] float2
-constexpr uint32_t kMmaSlotBytes = kMmaStV + 8 * 8 * kMmaVS;
+constexpr uint32_t kMmaStRow = kMmaStV + 8 * 8 * kMmaVS;                // int2: the y rows the batch reaches
+constexpr uint32_t kMmaSlotBytes = kMmaStRow + 16;
 static_assert(kMmaStV % 16 == 0 && kMmaSlotBytes % 16 == 0, "16-byte aligned staging");
 // Per instance: operand buffers, staged batches, and the offsets after B's buffers.  The plain
 // 3-D instance keeps three operand buffers -- A's third one takes the TMEM columns of the
@@ -404,6 +405,12 @@ __global__ void __launch_bounds__(mma_threads<KAHAN>(), KAHAN ? 1 : 2) k_spread_
                         wp[t * kMmaWS + lane] = (unsigned)(t - rs) < (unsigned)W ? wv : 0.f;
                     }
                 }
+                if constexpr (D == 3) {
+                    // first and last y row that some sample of the batch reaches
+                    const int lo = __reduce_min_sync(0xffffffffu, ok ? r[1] : kMmaTY);
+                    const int hi = __reduce_max_sync(0xffffffffu, ok ? r[1] + W - 1 : -1);
+                    if (lane == 0) *reinterpret_cast<int2 *>(sl + kMmaStRow) = make_int2(lo, hi);
+                }
                 float2 *vs = reinterpret_cast<float2 *>(sl + kMmaStV);
                 if (vec) {
 #pragma unroll
@@ -476,9 +483,23 @@ __global__ void __launch_bounds__(mma_threads<KAHAN>(), KAHAN ? 1 : 2) k_spread_
                 // A: cells (y, z) of this lane, samples SPW hk .. SPW hk + SPW - 1
                 const float4 *wy4 = reinterpret_cast<const float4 *>(sl + kMmaStWy) + (y * kMmaWS + SPW * hk) / 4;
                 const float4 *wz4 = reinterpret_cast<const float4 *>(sl + kMmaStWz) + (z * kMmaWS + SPW * hk) / 4;
+                // (3-D) this quarter's rows 2 q, 2 q + 1 that no sample of the batch reaches are
+                // zeros; the list's order by row makes that 32 % of all quarters
+                bool reach = true;
+                if constexpr (D == 3) {
+                    const int2 rows = *reinterpret_cast<const int2 *>(sl + kMmaStRow);
+                    reach = rows.x <= 2 * q + 1 && rows.y >= 2 * q;
+                }
 #pragma unroll
                 for (int h = 0; h < SPW / 8; ++h) {  // 8 samples at a time: fewer live registers
                     float hi[8], lo[8];
+                    if (!reach) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) hi[i] = 0.f;
+                        tmem_st_x8(tl + Cfg::a_col(buf) + SPW * hk + 8u * h, hi);
+                        tmem_st_x8(tl + Cfg::a_col(buf) + 32u + SPW * hk + 8u * h, hi);
+                        continue;
+                    }
 #pragma unroll
                     for (int i = 0; i < 2; ++i) {
                         const float4 p = wy4[2 * h + i], s = wz4[2 * h + i];
