@@ -211,6 +211,9 @@ int gbn_fft_band(gbn_plan *plan, void *grid, int direction, int band, gbn_stream
  * (nufft_func.py:751-764) */
 int gbn_pad_deapod(gbn_plan *plan, const void *img, gbn_layout img_layout, void *grid,
                    gbn_stream_t stream);
+/* gbn_pad_deapod followed by the transform of type 2: the grid that gbn_type2 interpolates
+ * (nufft_func.py:751-766) */
+int gbn_pad_fft(gbn_plan *plan, const void *img, gbn_layout img_layout, void *grid, gbn_stream_t stream);
 /* grid -> image with (1/M) (pi/tau)^(d/2) exp(tau|k|^2) / N (nufft_func.py:728-738) */
 int gbn_crop_deapod(gbn_plan *plan, const void *grid, void *img, gbn_layout img_layout,
                     gbn_stream_t stream);

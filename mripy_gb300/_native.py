@@ -23,7 +23,7 @@ EXPORTED = (
     "gbn_version", "gbn_status_string", "gbn_last_error", "gbn_grid_params",
     "gbn_plan_create", "gbn_plan_destroy", "gbn_plan_get_info", "gbn_plan_status", "gbn_plan_check_wait_expiry",
     "gbn_set_points", "gbn_plan_grid",
-    "gbn_spread", "gbn_interp", "gbn_fft", "gbn_fft_band", "gbn_pad_deapod", "gbn_crop_deapod",
+    "gbn_spread", "gbn_interp", "gbn_fft", "gbn_fft_band", "gbn_pad_deapod", "gbn_pad_fft", "gbn_crop_deapod",
     "gbn_type1", "gbn_type2", "gbn_type21",
     "gbn_sense_forward", "gbn_sense_adjoint", "gbn_sense_normal",
     "gbn_interp_grad_coords",
@@ -108,6 +108,7 @@ def _declare(lib):
         "gbn_fft": ([_vp, _vp, _i32, _vp], _i32),
         "gbn_fft_band": ([_vp, _vp, _i32, _i32, _vp], _i32),
         "gbn_pad_deapod": ([_vp, _vp, Layout, _vp, _vp], _i32),
+        "gbn_pad_fft": ([_vp, _vp, Layout, _vp, _vp], _i32),
         "gbn_crop_deapod": ([_vp, _vp, _vp, Layout, _vp], _i32),
         "gbn_type1": ([_vp, _vp, Layout, _vp, _vp, Layout, _vp], _i32),
         "gbn_type2": ([_vp, _vp, Layout, _vp, Layout, _vp], _i32),

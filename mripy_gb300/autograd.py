@@ -21,8 +21,6 @@ samples (M_total, n_coil) complex64.  The plan's trajectory groups are kept.
 """
 import torch
 
-from . import _native as N
-
 
 def _set_points(plan, coords):
     cs = [coords[d].detach().contiguous() for d in range(plan.dim)]
@@ -75,8 +73,7 @@ class _Type2(torch.autograd.Function):
         if ctx.needs_input_grad[0]:
             grad_img = _group_scale(plan, plan.type1(g), inverse=True)
         if ctx.needs_input_grad[1]:
-            grid = plan.pad_deapod(img)
-            plan.fft(grid, N.GBN_FFT_INVERSE if plan.iflag < 0 else N.GBN_FFT_FORWARD)
+            grid = plan.pad_fft(img)
             gx = plan.interp_grad_coords(grid, g)                   # (M, dim) float32
             grad_coords = gx.t().to(coords.dtype)
         return grad_img, grad_coords, None

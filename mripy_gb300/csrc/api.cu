@@ -312,18 +312,19 @@ int dir_type1(const gbn_plan *p) { return p->desc.iflag < 0 ? GBN_FFT_FORWARD : 
 int dir_type2(const gbn_plan *p) { return p->desc.iflag < 0 ? GBN_FFT_INVERSE : GBN_FFT_FORWARD; }
 
 // image (SENSE image and maps) -> deapodised, padded, transformed grid
-int image_to_grid(gbn_plan *p, const void *img, gbn_layout L, const void *sens, gbn_layout SL, cudaStream_t s) {
+int image_to_grid(gbn_plan *p, const void *img, gbn_layout L, const void *sens, gbn_layout SL, float2 *grid,
+                  cudaStream_t s) {
     const DeapodArgs a = deapod_args(p, false);
     const float2 *x = (const float2 *)img, *m = (const float2 *)sens;
     if (p->own_fft) {
-        GBN_CUDA(launch_band_fft_in(p->own, a, dir_type2(p) < 0 ? 0 : 1, x, L, m, SL, p->grid, s));
+        GBN_CUDA(launch_band_fft_in(p->own, a, dir_type2(p) < 0 ? 0 : 1, x, L, m, SL, grid, s));
         return GBN_OK;
     }
     if (m)
-        GBN_CUDA(launch_pad_sense(a, x, L, m, SL, p->grid, s));
+        GBN_CUDA(launch_pad_sense(a, x, L, m, SL, grid, s));
     else
-        GBN_CUDA(launch_pad(a, x, L, p->grid, s));
-    return fft_band_exec(p, p->grid, dir_type2(p), GBN_BAND_INPUT, s);
+        GBN_CUDA(launch_pad(a, x, L, grid, s));
+    return fft_band_exec(p, grid, dir_type2(p), GBN_BAND_INPUT, s);
 }
 
 // spread grid -> transformed, cropped, deapodised image (summed over the coils with the maps'
@@ -1000,10 +1001,12 @@ int plan_create_impl(const gbn_plan_desc *desc, gbn_plan **out) {
             reg_spread = false;
         }
     }
-    // 2-D with wide stencils, unless the caller chose a tile: 32 x 32 tiles in registers
-    if (p->dim == 2 && !tile_given && 2 * p->ns > 16) {
+    // 2-D with wide stencils or 1 to 3 coils, unless the caller chose a tile (or, below 18 taps,
+    // threads): 32 x 32 tiles in registers
+    if (p->dim == 2 && !tile_given && (2 * p->ns >= kWideMinW || desc->threads <= 0)) {
         Geom w{};
         w.dim = 2;
+        w.n_coil = (int)desc->n_coil;
         w.W = 2 * p->ns;
         for (int d = 0; d < 2; ++d) {
             w.nf[d] = p->nf[d];
@@ -1268,6 +1271,12 @@ int gbn_pad_deapod(gbn_plan *p, const void *img, gbn_layout L, void *grid, gbn_s
     return GBN_OK;
 }
 
+int gbn_pad_fft(gbn_plan *p, const void *img, gbn_layout L, void *grid, gbn_stream_t stream) {
+    GBN_TRY(check_plan(p, false));
+    if (!img || !grid) return fail(GBN_ERR_ARG, "null buffer");
+    return image_to_grid(p, img, L, nullptr, gbn_layout{}, (float2 *)grid, (cudaStream_t)stream);
+}
+
 int gbn_crop_deapod(gbn_plan *p, const void *grid, void *img, gbn_layout L, gbn_stream_t stream) {
     GBN_TRY(check_plan(p, true));
     if (!img || !grid) return fail(GBN_ERR_ARG, "null buffer");
@@ -1288,7 +1297,7 @@ int gbn_type2(gbn_plan *p, const void *img, gbn_layout il, void *c, gbn_layout c
     GBN_TRY(check_plan(p, true));
     if ((!c && p->M > 0) || !img) return fail(GBN_ERR_ARG, "null buffer");
     cudaStream_t s = (cudaStream_t)stream;
-    GBN_TRY(image_to_grid(p, img, il, nullptr, gbn_layout{}, s));
+    GBN_TRY(image_to_grid(p, img, il, nullptr, gbn_layout{}, p->grid, s));
     GBN_TRY(run_interp(p, p->grid, c, cl, nullptr, s));
     return GBN_OK;
 }
@@ -1299,7 +1308,7 @@ int gbn_type21(gbn_plan *p, const void *img, gbn_layout il, void *out, gbn_layou
     if (!img || !out) return fail(GBN_ERR_ARG, "null buffer");
     cudaStream_t s = (cudaStream_t)stream;
     const gbn_layout sl = {0, 1, p->desc.n_coil};
-    GBN_TRY(image_to_grid(p, img, il, nullptr, gbn_layout{}, s));
+    GBN_TRY(image_to_grid(p, img, il, nullptr, gbn_layout{}, p->grid, s));
     GBN_TRY(run_interp(p, p->grid, p->scratch.p, sl, dcf, s));
     GBN_TRY(run_spread(p, p->scratch.p, sl, nullptr, p->grid, s));
     return grid_to_image(p, out, ol, nullptr, gbn_layout{}, s);
@@ -1310,7 +1319,7 @@ int gbn_sense_forward(gbn_plan *p, const void *x, gbn_layout xl, const void *sen
     GBN_TRY(check_plan(p, true));
     if (!x || !sens || (!kdata && p->M > 0)) return fail(GBN_ERR_ARG, "null buffer");
     cudaStream_t s = (cudaStream_t)stream;
-    GBN_TRY(image_to_grid(p, x, xl, sens, sl, s));
+    GBN_TRY(image_to_grid(p, x, xl, sens, sl, p->grid, s));
     GBN_TRY(run_interp(p, p->grid, kdata, kl, nullptr, s));
     return GBN_OK;
 }
@@ -1330,7 +1339,7 @@ int gbn_sense_normal(gbn_plan *p, const void *x, gbn_layout xl, const void *sens
     if (!x || !sens || !x_out) return fail(GBN_ERR_ARG, "null buffer");
     cudaStream_t s = (cudaStream_t)stream;
     const gbn_layout scl = {0, 1, p->desc.n_coil};
-    GBN_TRY(image_to_grid(p, x, xl, sens, sl, s));
+    GBN_TRY(image_to_grid(p, x, xl, sens, sl, p->grid, s));
     GBN_TRY(run_interp(p, p->grid, p->scratch.p, scl, dcf, s));
     GBN_TRY(run_spread(p, p->scratch.p, scl, nullptr, p->grid, s));
     return grid_to_image(p, x_out, ol, sens, sl, s);

@@ -82,9 +82,10 @@ void few_tile(int n_coil, int tile[3]) {
     tile[2] = few_tz(n_coil);
 }
 
-// the wide-stencil 2-D spread applies: its tile, a grid of at least tile + stencil cells per axis
+// the one-coil-per-block 2-D register spread applies: stencils too wide for the other 2-D kernels,
+// or 1 to 3 coils; its tile, a grid of at least tile + stencil cells per axis
 bool spread_wide_applies(const Geom &g) {
-    return g.dim == 2 && g.W >= kWideMinW && g.W <= kWideMaxW && g.tile[0] == kWideTile && g.tile[1] == kWideTile &&
+    return g.dim == 2 && (g.W >= kWideMinW ? g.W <= kWideMaxW : g.n_coil <= kFewMaxCoils) && g.tile[0] == kWideTile && g.tile[1] == kWideTile &&
            g.nf[0] >= kWideTile + g.W && g.nf[1] >= kWideTile + g.W;
 }
 

@@ -351,6 +351,12 @@ class NufftPlan:
         N.check(self._lib.gbn_pad_deapod(self._h, _ptr(img), self._img_layout(img), _ptr(grid), _stream(stream)))
         return grid
 
+    def pad_fft(self, img, grid=None, stream=None):
+        """The grid that :meth:`type2` interpolates: padded, deapodised and transformed."""
+        grid = self.grid() if grid is None else grid
+        N.check(self._lib.gbn_pad_fft(self._h, _ptr(img), self._img_layout(img), _ptr(grid), _stream(stream)))
+        return grid
+
     def crop_deapod(self, grid, out=None, stream=None):
         self._check_points()
         out = self.empty_image() if out is None else out
