@@ -88,6 +88,7 @@ struct gbn_plan {
     int spread_variant = 0;  // 3-D, 8 coils: 0 library choice, 1 warp rows, 2 cubes, 3 tensor cores
     bool spread_items_interleaved = false;  // split tiles' work items interleave (cube kernel)
     int dense_min = kDenseDefault;  // 3-D spread tiles with this many samples use compensated sums (0: never)
+    const uint32_t *home_idx() const { return dup_idx.as<uint32_t>() + n_dup; }  // the sort's second list
     int64_t n_dense_sub = 0;
     bool rows_sorted = false;  // a tile's entries of the spread list are in the order of their y rows
     int64_t n_split = 0;  // spread tiles covered by more than one subproblem (listed in split_tiles)
@@ -128,8 +129,8 @@ struct gbn_plan {
     bool points_set = false;
     int64_t M = 0;
     std::vector<int64_t> traj_off;
-    DevBuf traj_off_d, grp_scale, pts, home_key, home_keys_sorted, touch_count, touch_off, counts,
-        iota, home_idx, home_pts, dup_keys, dup_vals, dup_keys_sorted, dup_idx, dup_pts, spread_tile_off,
+    DevBuf traj_off_d, grp_scale, pts, home_key, touch_count, touch_off, counts, home_pts,
+        dup_keys, dup_vals, dup_keys_sorted, dup_idx, dup_pts, spread_tile_off,
         home_tile_off, sub_off, sub_off_i, spread_subs, interp_subs, cub_tmp, scratch,
         stage_in, stage_out, stage_w, split_tiles, dense_subs;
     int64_t n_dup = 0, n_spread_sub = 0, n_interp_sub = 0;
@@ -526,7 +527,7 @@ int run_interp(gbn_plan *p, const float2 *grid, void *c, gbn_layout L, const flo
     a.g = p->gi;
     a.subs = p->interp_subs.as<int4>();
     a.pts = p->home_pts.as<float4>();
-    a.idx = p->home_idx.as<uint32_t>();
+    a.idx = p->home_idx();
     a.grid = grid;
     a.c = (float2 *)c;
     a.c_elem = L.elem_stride;
@@ -597,12 +598,9 @@ int set_points_impl(gbn_plan *p, int dtype, const void *x, const void *y, const 
     GBN_TRY(ensure(p, p->grp_scale, sizeof(float) * nt));
     GBN_TRY(ensure(p, p->pts, sizeof(float4) * Mb));
     GBN_TRY(ensure(p, p->home_key, sizeof(uint32_t) * Mb));
-    GBN_TRY(ensure(p, p->home_keys_sorted, sizeof(uint32_t) * Mb));
     GBN_TRY(ensure(p, p->touch_count, sizeof(uint32_t) * Mb));
     GBN_TRY(ensure(p, p->touch_off, sizeof(uint64_t) * Mb));
     GBN_TRY(ensure(p, p->counts, count_bytes));
-    GBN_TRY(ensure(p, p->iota, sizeof(uint32_t) * Mb));
-    GBN_TRY(ensure(p, p->home_idx, sizeof(uint32_t) * Mb));
     GBN_TRY(ensure(p, p->home_pts, sizeof(float4) * Mb));
     GBN_TRY(ensure(p, p->scratch, sizeof(float2) * Mb * (size_t)p->desc.n_coil));
     GBN_TRY(ensure(p, p->split_tiles, sizeof(uint32_t) * (size_t)std::max<int64_t>(Ts, 1)));
@@ -636,7 +634,6 @@ int set_points_impl(gbn_plan *p, int dtype, const void *x, const void *y, const 
     pa.traj_off = p->traj_off_d.as<int64_t>();
     pa.grp_scale = p->grp_scale.as<float>();
     pa.pts = p->pts.as<float4>();
-    pa.iota = p->iota.as<uint32_t>();
     pa.home_key = p->home_key.as<uint32_t>();
     pa.touch_count = p->touch_count.as<uint32_t>();
     pa.home_count = home_count;
@@ -678,8 +675,8 @@ int set_points_impl(gbn_plan *p, int dtype, const void *x, const void *y, const 
     }
     // The spread list (one entry per sample and tile its stencil reaches) has E = sum of the
     // touch counts entries.  When a bound on E fits kOneSyncEntries, its keys are written
-    // before E is known on the host, beside the home sort, so the round trip that brings E and
-    // the work-item counts back waits on no idle GPU.  Per axis a W-cell stencil reaches at
+    // before E is known on the host, so the round trip that brings E and the work-item counts
+    // back overlaps them.  Per axis a W-cell stencil reaches at
     // most ceil((W-1)/T) + 1 tiles, one more when a partial last tile sits at the wrap, and
     // never more than the axis has.
     uint64_t bound = (uint64_t)M;
@@ -691,25 +688,20 @@ int set_points_impl(gbn_plan *p, int dtype, const void *x, const void *y, const 
     const bool early = M > 0 && bound <= kOneSyncEntries;
     // the 3-D tensor-core kernels skip the y rows that none of a batch's samples reaches: a
     // tile's entries are sorted by their stencil's first row (one more radix pass of the sort)
-    const bool y_class = interp_mma_applies(p->gs, spread_cg(p)) && Ts < ((int64_t)1 << (32 - kYClassBits));
+    const bool y_class = interp_mma_applies(p->gs, spread_cg(p)) &&
+                         (Ts << kYClassBits) + Ti < ((int64_t)1 << 32);
     p->rows_sorted = y_class;
+    const uint32_t home_base = (uint32_t)Ts << (y_class ? kYClassBits : 0);  // above every spread key
     auto dup_keys = [&]() -> int {
         GBN_CUDA(launch_dup_keys(p->pts.as<float4>(), M, p->traj_off_d.as<int64_t>(), p->gs, to,
-                                 p->dup_keys.as<uint32_t>(), p->dup_vals.as<uint32_t>(), y_class, s));
+                                 p->dup_keys.as<uint32_t>(), p->dup_vals.as<uint32_t>(), y_class,
+                                 p->home_key.as<uint32_t>(), home_base, s));
         return GBN_OK;
     };
     if (early) {
-        GBN_TRY(ensure(p, p->dup_keys, sizeof(uint32_t) * (size_t)bound));
-        GBN_TRY(ensure(p, p->dup_vals, sizeof(uint32_t) * (size_t)bound));
+        GBN_TRY(ensure(p, p->dup_keys, sizeof(uint32_t) * (size_t)(bound + M)));
+        GBN_TRY(ensure(p, p->dup_vals, sizeof(uint32_t) * (size_t)(bound + M)));
         GBN_TRY(dup_keys());
-    }
-    if (M > 0) {
-        uint32_t *kin = p->home_key.as<uint32_t>(), *vin = p->iota.as<uint32_t>();
-        uint32_t *kout = p->home_keys_sorted.as<uint32_t>(), *vout = p->home_idx.as<uint32_t>();
-        const int bits = key_bits((uint64_t)Ti);
-        GBN_TRY(cub_call(p, [&](void *tmp, size_t &bytes) {
-            return cub::DeviceRadixSort::SortPairs(tmp, bytes, kin, kout, vin, vout, (int)M, 0, bits, s);
-        }));
     }
     TileTotals tot;
     GBN_CUDA(cudaMemcpyAsync(&tot, totals, sizeof(tot), cudaMemcpyDeviceToHost, s));
@@ -722,25 +714,27 @@ int set_points_impl(gbn_plan *p, int dtype, const void *x, const void *y, const 
         return fail(GBN_ERR_CAPACITY, "too many subproblems");
     p->n_dup = (int64_t)E;
     const size_t Eb = (size_t)std::max<uint64_t>(E, 1);
-    GBN_TRY(ensure(p, p->dup_keys, sizeof(uint32_t) * Eb));
-    GBN_TRY(ensure(p, p->dup_vals, sizeof(uint32_t) * Eb));
-    GBN_TRY(ensure(p, p->dup_keys_sorted, sizeof(uint32_t) * Eb));
-    GBN_TRY(ensure(p, p->dup_idx, sizeof(uint32_t) * Eb));
+    const size_t both = Eb + Mb;
+    GBN_TRY(ensure(p, p->dup_keys, sizeof(uint32_t) * both));
+    GBN_TRY(ensure(p, p->dup_vals, sizeof(uint32_t) * both));
+    GBN_TRY(ensure(p, p->dup_keys_sorted, sizeof(uint32_t) * both));
+    GBN_TRY(ensure(p, p->dup_idx, sizeof(uint32_t) * both));
     GBN_TRY(ensure(p, p->dup_pts, sizeof(float4) * Eb));
     GBN_TRY(ensure(p, p->spread_subs, sizeof(int4) * (size_t)std::max<uint64_t>(tot.spread_subs, 1)));
     GBN_TRY(ensure(p, p->interp_subs, sizeof(int4) * (size_t)std::max<uint64_t>(tot.interp_subs, 1)));
     GBN_TRY(ensure(p, p->dense_subs, sizeof(uint32_t) * (size_t)std::max<uint32_t>(tot.n_dense, 1)));
     if (!early && M > 0) GBN_TRY(dup_keys());
-    if (E > 0) {
+    if (M > 0) {
+        // stable, so each list keeps the samples of a bin (and row class) in their own order
         uint32_t *kin = p->dup_keys.as<uint32_t>(), *vin = p->dup_vals.as<uint32_t>();
         uint32_t *kout = p->dup_keys_sorted.as<uint32_t>(), *vout = p->dup_idx.as<uint32_t>();
-        const int bits = key_bits((uint64_t)Ts) + (y_class ? kYClassBits : 0);
+        const int bits = key_bits((uint64_t)home_base + (uint64_t)Ti);
         GBN_TRY(cub_call(p, [&](void *tmp, size_t &bytes) {
-            return cub::DeviceRadixSort::SortPairs(tmp, bytes, kin, kout, vin, vout, (int)E, 0, bits, s);
+            return cub::DeviceRadixSort::SortPairs(tmp, bytes, kin, kout, vin, vout, (int64_t)E + M, 0, bits, s);
         }));
     }
     GBN_CUDA(launch_gather_pts(p->pts.as<float4>(), p->dup_idx.as<uint32_t>(), (int64_t)E, p->dup_pts.as<float4>(),
-                               p->home_idx.as<uint32_t>(), M, p->home_pts.as<float4>(), s));
+                               p->home_idx(), M, p->home_pts.as<float4>(), s));
     js.split_list = p->split_tiles.as<uint32_t>();
     js.split_cursor = &totals->split_cursor;
     js.dense_list = p->dense_subs.as<uint32_t>();
@@ -1146,8 +1140,8 @@ int gbn_plan_destroy(gbn_plan *p) {
     if (p->kstatus) cudaFree(p->kstatus);
     for (int d = 0; d < 3; ++d)
         if (p->tab[d]) cudaFree(p->tab[d]);
-    DevBuf *bufs[] = {&p->traj_off_d, &p->grp_scale, &p->pts, &p->home_key, &p->home_keys_sorted,
-                      &p->touch_count, &p->touch_off, &p->counts, &p->iota, &p->home_idx, &p->home_pts,
+    DevBuf *bufs[] = {&p->traj_off_d, &p->grp_scale, &p->pts, &p->home_key,
+                      &p->touch_count, &p->touch_off, &p->counts, &p->home_pts,
                       &p->dup_keys, &p->dup_vals, &p->dup_keys_sorted, &p->dup_idx, &p->dup_pts,
                       &p->spread_tile_off, &p->home_tile_off, &p->sub_off, &p->sub_off_i,
                       &p->spread_subs, &p->interp_subs, &p->cub_tmp, &p->scratch, &p->stage_in,
@@ -1356,7 +1350,7 @@ int gbn_interp_grad_coords(gbn_plan *p, const void *grid, const void *grad_c, gb
     a.g = p->gi;
     a.subs = p->interp_subs.as<int4>();
     a.pts = p->home_pts.as<float4>();
-    a.idx = p->home_idx.as<uint32_t>();
+    a.idx = p->home_idx();
     a.grid = (const float2 *)grid;
     a.gc = (const float2 *)grad_c;
     a.c_elem = cl.elem_stride;

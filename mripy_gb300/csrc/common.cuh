@@ -108,13 +108,14 @@ struct PrepArgs {
     int64_t *traj_off;      // group offsets and scales (one group: written here)
     float *grp_scale;
     float4 *pts;
-    uint32_t *iota, *home_key, *touch_count;
+    uint32_t *home_key, *touch_count;
     uint32_t *home_count, *tile_count;  // zeroed: samples per interp bin, entries per spread tile
     uint32_t *status;                   // zeroed: bit 0 set by a coordinate that is not finite
 };
 cudaError_t launch_prep(int coord_dtype, PrepArgs a, cudaStream_t s);
 cudaError_t launch_dup_keys(const float4 *pts, int64_t M, const int64_t *d_traj_off, const Geom &gs,
-                            const uint64_t *touch_off, uint32_t *keys, uint32_t *vals, bool y_class, cudaStream_t s);
+                            const uint64_t *touch_off, uint32_t *keys, uint32_t *vals, bool y_class,
+                            const uint32_t *home_key, uint32_t home_base, cudaStream_t s);
 constexpr int kYClassBits = 5;  // W + tile rows - 1 <= 16 + 8 - 1 classes
 // out[i] = pts[idx[i]] for both lists
 cudaError_t launch_gather_pts(const float4 *pts, const uint32_t *idx, int64_t n, float4 *out, const uint32_t *idx2,

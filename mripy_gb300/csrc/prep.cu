@@ -96,7 +96,6 @@ __global__ void __launch_bounds__(256) k_prep(PrepArgs a) {
         for (int d = 0; d < 3; ++d) { f[d] = 0.f; c0[d] = 0; }
     }
     a.pts[j] = make_float4(f[0], f[1], f[2], __uint_as_float(pack_cells(dim, c0[0], c0[1], c0[2])));
-    a.iota[j] = (uint32_t)j;
 
     const int g = gs.n_traj == 1 ? 0 : group_of(a.traj_off, gs.n_traj, j);
     int t[3] = {0, 0, 0}, n[3] = {1, 1, 1}, t0[3] = {0, 0, 0};
@@ -129,10 +128,12 @@ __global__ void __launch_bounds__(256) k_prep(PrepArgs a) {
 
 // The (sample, tile) entries, each sample's adjacent.  y_class: the key's low kYClassBits hold
 // the stencil's first y row in the tile (+ W - 1: 0 is a stencil that reaches row 0 only), so
-// that the sort leaves a tile's samples in the order of the rows they reach.
+// that the sort leaves a tile's samples in the order of the rows they reach.  Before them, one
+// entry per sample with its home bin's key above all of theirs: one sort makes both lists.
 __global__ void k_dup_keys(const float4 *__restrict__ pts, int64_t M, const int64_t *__restrict__ traj_off,
                            Geom gs, const uint64_t *__restrict__ touch_off, uint32_t *__restrict__ keys,
-                           uint32_t *__restrict__ vals, int y_class) {
+                           uint32_t *__restrict__ vals, int y_class,
+                           const uint32_t *__restrict__ home_key, uint32_t home_base) {
     int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (j >= M) return;
     const int dim = gs.dim;
@@ -146,7 +147,9 @@ __global__ void k_dup_keys(const float4 *__restrict__ pts, int64_t M, const int6
         t0[d] = c0[d] / gs.tile[d];
     }
     const uint32_t base = gs.n_traj == 1 ? 0u : (uint32_t)group_of(traj_off, gs.n_traj, j) * (uint32_t)gs.ntiles;
-    uint64_t pos = touch_off[j];
+    keys[j] = home_base + home_key[j];
+    vals[j] = (uint32_t)j;
+    uint64_t pos = (uint64_t)M + touch_off[j];
     for (int a = 0; a < n[0]; ++a) {
         int ta = (t0[0] + a) % gs.ntile[0];
         for (int b = 0; b < n[1]; ++b) {
@@ -306,9 +309,11 @@ cudaError_t launch_prep(int coord_dtype, PrepArgs a, cudaStream_t s) {
 }
 
 cudaError_t launch_dup_keys(const float4 *pts, int64_t M, const int64_t *d_traj_off, const Geom &gs,
-                            const uint64_t *touch_off, uint32_t *keys, uint32_t *vals, bool y_class, cudaStream_t s) {
+                            const uint64_t *touch_off, uint32_t *keys, uint32_t *vals, bool y_class,
+                            const uint32_t *home_key, uint32_t home_base, cudaStream_t s) {
     if (M == 0) return cudaSuccess;
-    k_dup_keys<<<blocks_for(M, 256), 256, 0, s>>>(pts, M, d_traj_off, gs, touch_off, keys, vals, y_class ? 1 : 0);
+    k_dup_keys<<<blocks_for(M, 256), 256, 0, s>>>(pts, M, d_traj_off, gs, touch_off, keys, vals, y_class ? 1 : 0,
+                                                  home_key, home_base);
     return cudaGetLastError();
 }
 
