@@ -833,7 +833,7 @@ int make_own_fft(gbn_plan *p) {
         if (!p->own.e[d]) return GBN_OK;
     }
     // blocks of the widest launch
-    if ((double)p->n_inst * p->nf[0] * std::max(p->nf[1], 16) / 16 * std::max(p->nf[2], 16) / 8 > 2e9) return GBN_OK;
+    if ((double)p->n_inst * p->nf[0] * std::max(p->nf[1], 16) / 8 * std::max(p->nf[2], 16) / 8 > 2e9) return GBN_OK;
     size_t cells = 0;
     for (int d = 0; d < p->dim; ++d) cells += (size_t)p->nf[d];
     GBN_CUDA(cudaMalloc((void **)&p->own_tw, sizeof(float2) * cells));

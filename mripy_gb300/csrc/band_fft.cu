@@ -73,7 +73,7 @@ cudaError_t strided(const BandFft &b, const DeapodArgs &a, int d, bool out, int 
         c.sub_skip = p.nf - p.m;
         c.sub_stride = (int64_t)g.nf[1] * g.nf[2];
     }
-    c.chunks = (c.cols + kFftLines - 1) / kFftLines;
+    c.chunks = (c.cols + b.e[d]->lines - 1) / b.e[d]->lines;
     const int64_t blocks = (int64_t)g.n_coil * g.n_traj * c.n_sub * c.chunks;
     return b.e[d]->cols(grid, c, blocks, out, s);
 }

@@ -189,13 +189,19 @@ GBN_DFT(32, 8, 4);
 
 // ------------------------------------------------------------------ geometry
 
-template <int R1, int R2> struct FftLine {
-    static constexpr int N = R1 * R2;
+// Lines per block of a strided pass: 8 for the lengths with a radix above 18, whose cells take so
+// many registers that only more, smaller blocks overlap their phases (384: 318 -> 285 us for
+// 768 grids of 384^2); else 16 (with 8: 162 cells 81 -> 92 us, whose rows start off 64-byte
+// boundaries; 256 unchanged).
+constexpr int fft_cols(int r1, int r2) { return r1 > 18 || r2 > 18 ? 8 : 16; }
+
+template <int R1, int R2, int LINES = kFftLines> struct FftLine {
+    static constexpr int N = R1 * R2, LN = LINES;
     static constexpr int J = R1 < R2 ? R1 : R2;   // threads per line
-    static constexpr int T = kFftLines * J;
+    static constexpr int T = LINES * J;
     static constexpr int P = R1 + 1;              // exchange: output r of butterfly j at j P + r
     static constexpr int PITCH = (R2 * P) | 1;    // odd: adjacent lines on distinct banks
-    static constexpr size_t SMEM = (size_t)kFftLines * PITCH * sizeof(float2);
+    static constexpr size_t SMEM = (size_t)LINES * PITCH * sizeof(float2);
     static constexpr int MAXR = R1 > R2 ? R1 : R2;
     // resident blocks the register budgets are set for.  Measured (256^3 grids, strided passes):
     // band in 3 blocks 0.46 ms against 2 blocks 0.57; band out 0.53 against 0.46.
@@ -221,14 +227,14 @@ __device__ __forceinline__ void fft_second(const float2 *line, int k, const floa
 // OUT: only the band's cells are written (before a crop); else only the band's cells are read
 // and the others are zero (after a pad).
 template <int R1, int R2, bool OUT>
-__global__ void __launch_bounds__(FftLine<R1, R2>::T, OUT ? FftLine<R1, R2>::BLOCKS_OUT : FftLine<R1, R2>::BLOCKS_IN)
+__global__ void __launch_bounds__(FftLine<R1, R2, fft_cols(R1, R2)>::T, OUT ? FftLine<R1, R2, fft_cols(R1, R2)>::BLOCKS_OUT : FftLine<R1, R2, fft_cols(R1, R2)>::BLOCKS_IN)
     k_fft_cols(float2 *__restrict__ grid, FftCols a) {
-    using L = FftLine<R1, R2>;
+    using L = FftLine<R1, R2, fft_cols(R1, R2)>;
     extern __shared__ float2 sm_fft[];
     const int ch = blockIdx.x % a.chunks, ob = blockIdx.x / a.chunks;
     const int inst = ob / a.n_sub, sub = ob - inst * a.n_sub;
-    const int l = threadIdx.x % kFftLines, jt = threadIdx.x / kFftLines;
-    const int col = ch * kFftLines + l;
+    const int l = threadIdx.x % L::LN, jt = threadIdx.x / L::LN;
+    const int col = ch * L::LN + l;
     const bool live = col < a.cols;
     // sub-volumes (the band planes of the axis in front) at the two ends of that axis
     const int64_t so = sub < a.sub_lo ? sub : sub + a.sub_skip;
@@ -495,8 +501,9 @@ struct FftLaunch {
         return e;
     }
     static cudaError_t cols(float2 *grid, const FftCols &a, int64_t blocks, bool out, cudaStream_t s) {
-        if (out) k_fft_cols<R1, R2, true><<<(unsigned)blocks, L::T, L::SMEM, s>>>(grid, a);
-        else k_fft_cols<R1, R2, false><<<(unsigned)blocks, L::T, L::SMEM, s>>>(grid, a);
+        using C = FftLine<R1, R2, fft_cols(R1, R2)>;
+        if (out) k_fft_cols<R1, R2, true><<<(unsigned)blocks, C::T, C::SMEM, s>>>(grid, a);
+        else k_fft_cols<R1, R2, false><<<(unsigned)blocks, C::T, C::SMEM, s>>>(grid, a);
         return cudaGetLastError();
     }
     static cudaError_t rows(float2 *grid, const FftRows &a, int64_t blocks, int kind, cudaStream_t s) {
@@ -505,7 +512,7 @@ struct FftLaunch {
         else k_fft_rows_sense<R1, R2><<<(unsigned)blocks, L::T, L::SMEM, s>>>(a, grid);
         return cudaGetLastError();
     }
-    static FftEntry entry() { return FftEntry{R1 * R2, prepare, cols, rows}; }
+    static FftEntry entry() { return FftEntry{R1 * R2, fft_cols(R1, R2), prepare, cols, rows}; }
 };
 
 }  // namespace gbn

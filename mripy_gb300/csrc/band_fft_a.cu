@@ -11,6 +11,6 @@ const FftEntry fft_a[] = {
     FftLaunch<8, 12>::entry(),
     FftLaunch<10, 10>::entry(),
     FftLaunch<9, 12>::entry(),
-    FftEntry{0, nullptr, nullptr, nullptr}};
+    FftEntry{0, 0, nullptr, nullptr, nullptr}};
 
 }  // namespace gbn

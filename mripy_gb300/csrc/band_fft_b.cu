@@ -12,6 +12,6 @@ const FftEntry fft_b[] = {
     FftLaunch<10, 15>::entry(),
     FftLaunch<10, 16>::entry(),
     FftLaunch<9, 18>::entry(),
-    FftEntry{0, nullptr, nullptr, nullptr}};
+    FftEntry{0, 0, nullptr, nullptr, nullptr}};
 
 }  // namespace gbn

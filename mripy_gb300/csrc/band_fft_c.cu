@@ -12,6 +12,6 @@ const FftEntry fft_c[] = {
     FftLaunch<12, 18>::entry(),
     FftLaunch<14, 16>::entry(),
     FftLaunch<20, 32>::entry(),
-    FftEntry{0, nullptr, nullptr, nullptr}};
+    FftEntry{0, 0, nullptr, nullptr, nullptr}};
 
 }  // namespace gbn

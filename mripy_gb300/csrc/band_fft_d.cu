@@ -11,6 +11,6 @@ const FftEntry fft_d[] = {
     FftLaunch<16, 18>::entry(),
     FftLaunch<15, 20>::entry(),
     FftLaunch<24, 24>::entry(),
-    FftEntry{0, nullptr, nullptr, nullptr}};
+    FftEntry{0, 0, nullptr, nullptr, nullptr}};
 
 }  // namespace gbn

@@ -11,6 +11,6 @@ const FftEntry fft_e[] = {
     FftLaunch<18, 20>::entry(),
     FftLaunch<16, 24>::entry(),
     FftLaunch<24, 32>::entry(),
-    FftEntry{0, nullptr, nullptr, nullptr}};
+    FftEntry{0, 0, nullptr, nullptr, nullptr}};
 
 }  // namespace gbn

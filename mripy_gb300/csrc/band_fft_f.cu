@@ -9,6 +9,6 @@ const FftEntry fft_f[] = {
     FftLaunch<18, 24>::entry(),
     FftLaunch<20, 24>::entry(),
     FftLaunch<16, 32>::entry(),
-    FftEntry{0, nullptr, nullptr, nullptr}};
+    FftEntry{0, 0, nullptr, nullptr, nullptr}};
 
 }  // namespace gbn

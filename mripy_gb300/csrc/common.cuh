@@ -273,10 +273,10 @@ cudaError_t launch_crop_sense(const DeapodArgs &a, const float2 *grid, const flo
                               gbn_layout SL, float2 *x, gbn_layout XL, cudaStream_t s);
 
 // band_fft.cuh: transforms with pad and crop fused in
-constexpr int kFftLines = 16;  // lines per block
+constexpr int kFftLines = 16;  // lines per block of the row passes
 struct FftCols {               // one strided axis, in place
     int64_t G, stride;         // cells per instance; cells between neighbours along the axis
-    int cols, chunks;          // inner cells, blocks of kFftLines of them
+    int cols, chunks;          // inner cells, blocks of FftEntry::lines of them
     int n_sub, sub_lo;         // sub-volumes per instance: 0 .. sub_lo - 1, then those after
     int64_t sub_skip, sub_stride;  // sub_skip further ones
     int lo, hi;                // the axis' band: cells [0, lo) and [N - hi, N)
@@ -302,7 +302,7 @@ struct FftRows {               // the contiguous axis, between image and grid
     gbn_layout SL;
 };
 struct FftEntry {              // the kernels of one length
-    int n;
+    int n, lines;              // lines per block of the strided passes
     cudaError_t (*prepare)();  // raises their shared-memory limits
     cudaError_t (*cols)(float2 *grid, const FftCols &a, int64_t blocks, bool out, cudaStream_t s);
     cudaError_t (*rows)(float2 *grid, const FftRows &a, int64_t blocks, int kind, cudaStream_t s);
