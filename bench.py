@@ -405,6 +405,7 @@ def run_gpu(args, wl):
     t_interp, _ = event_time(torch, lambda: plan.interp(grid_copy, out=samples), reps, stream, flush)
     t_spread, _ = event_time(torch, lambda: plan.spread(samples, grid), reps, stream, flush)
     t_pad, _ = event_time(torch, lambda: plan.pad_deapod(img, grid), reps, stream, flush)
+    t_padfft, _ = event_time(torch, lambda: plan.pad_fft(img, grid), reps, stream, flush)
     # the step's transforms: pruned to the image band where the plan says so (fft_variant 2)
     t_fft, _ = event_time(torch, lambda: plan.fft_band(grid, N.GBN_FFT_FORWARD, N.GBN_BAND_INPUT), reps, stream, flush)
     t_fft_inv, _ = event_time(torch, lambda: plan.fft_band(grid, N.GBN_FFT_INVERSE, N.GBN_BAND_OUTPUT), reps, stream,
@@ -459,8 +460,12 @@ def run_gpu(args, wl):
                      "measured max SM clock"}
     if info.get("interp_variant") == 2:
         # the tensor-core interp: per (sample, tile) pair 3 TF32 MMAs' worth of M = 128
-        # samples x N = 64 over K = 128 (y, z) cells, as the spread
-        mma_flop_i = info["spread_entries"] * 3 * 2 * 128 * 64
+        # samples x N = 64 over the K = 32 (y, z) cells of each pair of y rows that its stencil
+        # reaches (a batch issues those that any of its samples reaches: slightly more)
+        W = 2 * info["nspread"]
+        rows = [(max(r, 0) // 2, min(r + W - 1, 7) // 2) for r in range(1 - W, 8)]
+        reached = sum(hi - lo + 1 for lo, hi in rows) / (4 * len(rows))
+        mma_flop_i = info["spread_entries"] * 3 * 2 * 128 * 64 * reached
         result["roofline"]["interp_tensor"] = {
             "kernel": "k_interp3d_mma", "mma_tflop_per_launch": round(mma_flop_i / 1e12, 3),
             "achieved_tflops": round(mma_flop_i / (t_interp * 1e-3) / 1e12, 1),
@@ -483,11 +488,15 @@ def run_gpu(args, wl):
     result["kernels_ms"] = {"interp": round(t_interp, 4), "spread": round(t_spread, 4), "pad_deapod": round(t_pad, 4),
                             "fft": round(t_fft, 4), "fft_inverse": round(t_fft_inv, 4),
                             "fft_full_transform": round(t_fft_full, 4), "crop_deapod": round(t_crop, 4),
-                            "fft_pruned_to_band": info["fft_variant"] == 2}
+                            "fft_pruned_to_band": info["fft_variant"] == 2,
+                            "step_runs": ("band transforms with pad and crop fused in (one call each way: "
+                                          "%.4f ms in); the pad, fft and crop entries are the separate stage calls"
+                                          % t_padfft if info["band_fft"] else "the pad, fft and crop stages")}
     # this library's kernels per step (cuFFT and memsets not counted): pad, interp, crop and
     # what the spread launched in the eager step before capture (split-tile zeroing unless the
     # grid is cleared by a memset; the 3-D compensated instance for dense tiles)
-    per_step = 2 + (1 if info["interp_subproblems"] else 0) + plan.info()["spread_kernels"]
+    # (with the band transforms: their passes, one per axis and direction, instead of pad and crop)
+    per_step = (2 * wl.dim if info["band_fft"] else 2) + (1 if info["interp_subproblems"] else 0) + plan.info()["spread_kernels"]
     result["gpu_launches"] = per_step * args.steps
 
     # --- plain per-instance path: single-coil plan per group, eager, instance by instance

@@ -98,14 +98,12 @@ typedef struct {
                                    the spread's tiles allow (per tile a TF32 GEMM over the
                                    tile's samples, partial sums added with float atomics) */
     int32_t fft_variant;        /* FFT of the composite calls (type 1/2/21, SENSE): 0 = library
-                                   choice (pruned on 3-D grids of >= 2^21 cells per instance,
-                                   <= 256 instances; the full transform if cuFFT cannot make
-                                   the pruned plans), 1 = the full transform, 2 = pruned
-                                   wherever the image band is narrower than the grid (2-D and
-                                   3-D, <= 4096 instances).  Pruned: the trailing axes are
-                                   transformed only on the grid planes inside the image band
-                                   along x, which hold every non-zero cell of the pad and
-                                   every cell the crop reads (see gbn_fft_band) */
+                                   choice (2-D and 3-D grids whose every length is supported:
+                                   band transforms with pad, deapodisation and crop fused in;
+                                   else pruned on 3-D grids of >= 2^21 cells per instance,
+                                   <= 256 instances; else the full transform), 1 = the full
+                                   transform, 2 = pruned wherever the image band is narrower
+                                   than the grid (at most 4096 instances) */
 } gbn_plan_desc;
 
 typedef struct {
@@ -135,7 +133,9 @@ typedef struct {
     int32_t interp_variant;    /* 2 when the interp runs on the tensor cores (3-D, 8 coils per
                                   group; partial sums added with float atomics, so the
                                   samples agree run to run to rounding), else 1 */
-    int32_t fft_variant;       /* 2 when the composite calls run the pruned transform, else 1 */
+    int32_t fft_variant;       /* 2 where gbn_fft_band is the pruned transform, else 1 */
+    int32_t band_fft;          /* 1 when the composite calls run transforms with pad, deapodisation
+                                  and crop fused in (fft_variant 0 and supported grid lengths) */
 } gbn_plan_info;
 
 /* element strides (in complex64 elements) of a strided complex array */

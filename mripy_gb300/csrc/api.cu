@@ -1217,6 +1217,7 @@ int gbn_plan_get_info(const gbn_plan *p, gbn_plan_info *o) {
     o->spread_variant = spread_path_kind(p->gs, spread_cg(p), p->spread_variant, p->threads);
     o->interp_variant = interp_on_tensor_cores(p) ? 2 : 1;
     o->fft_variant = p->fft_band ? 2 : 1;
+    o->band_fft = p->own_fft ? 1 : 0;
     o->device_bytes = (int64_t)p->device_bytes;
     return GBN_OK;
 }

@@ -77,9 +77,10 @@ template <bool KAHAN> constexpr int mma_builders() { return KAHAN ? 16 : 8; }
 // with its own operand buffer
 template <int D, bool KAHAN> constexpr int mma_groups() { return D == 3 && !KAHAN ? 2 : 1; }
 template <bool KAHAN> constexpr int mma_threads() { return 32 * (mma_builders<KAHAN>() + kMmaLoaders + 1); }
-constexpr uint32_t kMmaTmemCols = 256;              // A (hi, lo) x 2 buffers: 0..127; D, S: 128..255
+// A (hi, lo) x 2 buffers: 0..127; D from 128; then A's third buffer (3-D) or the running sum S of
+// the drained accumulators (2-D)
+constexpr uint32_t kMmaTmemCols = 256;
 constexpr uint32_t kMmaColD = 128;                  // the MMAs' accumulator
-constexpr uint32_t kMmaColS = 192;                  // the running sum of the drained accumulators (3-D)
 // the compensated instance: two accumulators D (batch k in D[k % 2]), the running sum S, its
 // Kahan compensation C and the current group's FP32 sum G; one block per SM
 constexpr uint32_t kMmaTmemColsK = 512;

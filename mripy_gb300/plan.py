@@ -183,7 +183,7 @@ class NufftPlan:
             "dense_subproblems": inf.dense_subproblems,
             "spread_kernels": inf.spread_kernels, "split_tiles": inf.split_tiles,
             "spread_variant": inf.spread_variant, "interp_variant": inf.interp_variant,
-            "fft_variant": inf.fft_variant,
+            "fft_variant": inf.fft_variant, "band_fft": inf.band_fft,
         }
 
     def status(self, stream=None):
