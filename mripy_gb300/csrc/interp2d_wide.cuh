@@ -16,9 +16,12 @@ namespace gbn {
 
 // 16-byte units per staged row
 __host__ __device__ inline int wide_row_units(const Geom &g) { return (g.tile[1] + g.W - 1 + 2) / 2; }
+// One unit more than the window: the lane past a sample's last tap (its weights are zero) reads
+// the unit behind the row where the sample is in the last cell of an even tile whose window
+// starts on an odd cell.
 inline size_t interp2d_wide_smem(const Geom &g) {
     if (g.dim != 2 || g.W < kWideMinW || g.W > kWideMaxW) return 0;
-    return (size_t)(g.tile[0] + g.W - 1) * wide_row_units(g) * sizeof(float4);
+    return ((size_t)(g.tile[0] + g.W - 1) * wide_row_units(g) + 1) * sizeof(float4);
 }
 
 __global__ void __launch_bounds__(256) k_interp2d_wide(InterpArgs a, int vec) {

@@ -35,9 +35,13 @@ __host__ __device__ inline int one_row_units(const Geom &g) {
     if (g.W == 10) r = ((r + 6) & ~7) + 1;
     return r;
 }
+// One unit more than the window: a sample in the last cell of an even tile whose window starts
+// on an odd cell has its W / 2 lanes end the row, and the lane past them (its weights are zero)
+// reads the unit behind it.  (Sending that lane to the sample's first unit instead: 20 density
+// iterations of 768,000 samples 16.1 ms against 15.1.)
 inline size_t interp3d_one_smem_bytes(const Geom &g) {
     if (g.dim != 3 || g.W > kOneMaxW || (g.W & 1)) return 0;
-    return (size_t)(g.tile[0] + g.W - 1) * (g.tile[1] + g.W - 1) * one_row_units(g) * sizeof(float4);
+    return ((size_t)(g.tile[0] + g.W - 1) * (g.tile[1] + g.W - 1) * one_row_units(g) + 1) * sizeof(float4);
 }
 
 template <int WT>

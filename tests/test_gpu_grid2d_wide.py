@@ -109,3 +109,18 @@ def test_wide_unaligned_grid_and_non_finite():
     assert touched[7, 0] and touched.sum() < 400
     assert np.array_equal(k1[~touched], k0[~touched])
     p.close()
+
+
+@pytest.mark.parametrize("eps,ns", [(6e-9, 9), (2e-13, 12), (1e-15, 14), (1e-16, 15)])
+def test_wide_interp_samples_in_every_cell_of_a_bin(eps, ns):
+    """Samples in the bins' last cells, where the lane past the last tap would read behind the
+    window (even tiles whose window starts on an odd cell)."""
+    rng = np.random.default_rng(ns)
+    M, shape = 20000, (20, 20)
+    xs = rng.uniform(-np.pi, np.pi, (2, M))
+    p = NufftPlan(2, shape, eps=eps).set_points([cuda(v) for v in xs])
+    nsp, nf, tau = O.grid_params(2, *shape, eps=eps)
+    assert nsp == ns
+    G = cvec(rng, (1,) + nf)
+    assert rel(p.interp(cuda(G)), np.prod(nf) * O.interp(tuple(xs), G, tau, nsp).T) < TOL_REF
+    p.close()

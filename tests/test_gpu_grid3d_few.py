@@ -155,3 +155,18 @@ def test_few_coils_real_samples_match_complex():
     w = w.real.cpu().numpy()[:, 0]
     assert rel(d, w * M / w.sum()) < TOL_REF
     p.close()
+
+
+@pytest.mark.parametrize("eps,ns", [(1e-3, 3), (1e-4, 4), (1e-5, 5), (5e-6, 6), (1e-6, 7)])
+def test_one_coil_interp_samples_in_every_cell_of_a_bin(eps, ns):
+    """Staged bins with samples in their last cells, where the lane past the last tap would read
+    behind the window (even tiles whose window starts on an odd cell)."""
+    rng = np.random.default_rng(ns)
+    M, shape = 30000, (16, 16, 16)
+    xs = rng.uniform(-np.pi, np.pi, (3, M))
+    p = NufftPlan(3, shape, eps=eps).set_points([cuda(v) for v in xs])
+    nsp, nf, tau = O.grid_params(3, *shape, eps=eps)
+    assert nsp == ns and M > 64 * p.info()["interp_subproblems"]
+    G = cvec(rng, (1,) + nf)
+    assert rel(p.interp(cuda(G)), np.prod(nf) * O.interp(tuple(xs), G, tau, nsp).T) < TOL_REF
+    p.close()
