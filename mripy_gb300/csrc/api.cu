@@ -505,7 +505,9 @@ bool interp_on_tensor_cores(const gbn_plan *p) {
            (p->rows_sorted || !p->points_set);
 }
 
-int run_interp(gbn_plan *p, const float2 *grid, void *c, gbn_layout L, const float *weight, cudaStream_t s) {
+// real: the grid's imaginary parts are zero, and the samples' come out as zero
+int run_interp(gbn_plan *p, const float2 *grid, void *c, gbn_layout L, const float *weight, cudaStream_t s,
+               bool real = false) {
     NvtxRange range("gbn interp");
     if (interp_on_tensor_cores(p)) {
         MmaInterpArgs m;
@@ -533,6 +535,7 @@ int run_interp(gbn_plan *p, const float2 *grid, void *c, gbn_layout L, const flo
     a.c_elem = L.elem_stride;
     a.c_coil = L.coil_stride;
     a.weight = weight;
+    a.real = real && p->M >= kRealMinBin * p->n_interp_sub ? 1 : 0;
     const int cg = interp_cg(p);
     // 2-D: windows staged by tensor copies when the grid admits a tensor map
     TmaWin t{};
@@ -1572,7 +1575,7 @@ int gbn_dcf_pipe_menon(gbn_plan *p, int32_t n_iter, float *dcf, gbn_stream_t str
     GBN_CUDA(launch_dcf_fill(w, p->M, s));
     for (int it = 0; it < n_iter; ++it) {
         GBN_TRY(run_spread(p, w, cl, nullptr, p->grid, s, true));  // real weights
-        GBN_TRY(run_interp(p, p->grid, cw, cl, nullptr, s));
+        GBN_TRY(run_interp(p, p->grid, cw, cl, nullptr, s, true));
         GBN_CUDA(launch_dcf_update(w, cw, p->M, s));
     }
     GBN_CUDA(launch_dcf_finish(w, p->traj_off_d.as<int64_t>(), p->desc.n_traj, partial, dcf, s));

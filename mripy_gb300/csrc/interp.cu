@@ -16,6 +16,7 @@
 #include "interp2d_wide.cuh"
 #include "interp3d_mma.cuh"
 #include "interp3d_one.cuh"
+#include "interp3d_real.cuh"
 
 namespace gbn {
 
@@ -115,6 +116,17 @@ cudaError_t launch_interp(const InterpArgs &a, int64_t n_sub, int coil_group, in
             return launch_interp3d_planes(a, n_sub, coil_group, th, nullptr, nullptr, s);
         if (coil_group == 1 && interp3d_one_applies(a.g)) {
             const int vec = (uintptr_t)a.grid % 16 == 0 && a.g.nf[2] % 2 == 0 && a.g.G % 2 == 0;
+            const size_t rsmem = interp3d_real_smem_bytes(a.g);
+            if (a.real && vec && rsmem > 0 && rsmem <= 112 * 1024) {
+                auto kern = a.g.W == 6   ? k_interp3d_real<6>
+                            : a.g.W == 8 ? k_interp3d_real<8>
+                            : a.g.W == 10 ? k_interp3d_real<10>
+                                          : k_interp3d_real<12>;
+                err = set_smem(kern, rsmem);
+                if (err != cudaSuccess) return err;
+                kern<<<grid, th, rsmem, s>>>(a);
+                return cudaGetLastError();
+            }
             GBN_DISPATCH_W(a.g.W, {
                 auto kern = k_interp3d_one<WT>;
                 err = set_smem(kern, smem);
