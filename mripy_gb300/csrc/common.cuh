@@ -221,7 +221,7 @@ bool interp_wide_applies(const Geom &g);
 int spread_kernel_count(const SpreadArgs &a, int64_t n_sub, int coil_group, int threads);
 // interps of a real grid take k_interp3d_real from this many samples a bin on the average: it
 // stages every bin's window.  Measured, 20 density iterations, 10 taps, complex -> real interp:
-// 84 samples a bin 15.11 -> 13.83 ms, 35 a bin 7.33 -> 7.04, 15 a bin 4.17 -> 4.43.
+// 84 samples a bin 14.83 -> 13.81 ms, 35 a bin 7.13 -> 7.04, 15 a bin 4.07 -> 4.43.
 constexpr int kRealMinBin = 24;
 cudaError_t launch_interp(const InterpArgs &a, int64_t n_sub, int coil_group, int threads,
                           cudaStream_t s);

@@ -127,15 +127,15 @@ cudaError_t launch_interp(const InterpArgs &a, int64_t n_sub, int coil_group, in
                 kern<<<grid, th, rsmem, s>>>(a);
                 return cudaGetLastError();
             }
-            GBN_DISPATCH_W(a.g.W, {
-                auto kern = k_interp3d_one<WT>;
-                err = set_smem(kern, smem);
-                if (err == cudaSuccess) {
-                    kern<<<grid, th, smem, s>>>(a, vec);
-                    err = cudaGetLastError();
-                }
-            });
-            return err;
+            auto kern = a.g.W == 6    ? k_interp3d_one<6>
+                        : a.g.W == 8  ? k_interp3d_one<8>
+                        : a.g.W == 10 ? k_interp3d_one<10>
+                        : a.g.W == 12 ? k_interp3d_one<12>
+                                      : k_interp3d_one<0>;
+            err = set_smem(kern, smem);
+            if (err != cudaSuccess) return err;
+            kern<<<grid, th, smem, s>>>(a, vec);
+            return cudaGetLastError();
         }
         const size_t wsmem = interp3d_smem_bytes(a.g, coil_group);  // the whole staged window
         GBN_DISPATCH_W(a.g.W, GBN_DISPATCH_CG(coil_group, {

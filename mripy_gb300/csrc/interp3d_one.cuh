@@ -14,6 +14,9 @@
 // (mod 8), and a step takes the rows {0, 6, 4, 2, 8} + step: their 6-unit runs then start at
 // units 0, 6, 12, 18, 24 (mod 8), i.e. the warp's units are consecutive mod 8 and no quarter
 // warp conflicts.
+// Lanes without taps (2 of 32 there, up to 3 of 8 in the 8-lane rows) repeat the first unit of
+// their own row.  Sent to the sample's first unit instead they conflict with their quarter
+// warp: 768,000 samples 0.385 -> 0.373 ms at 10 taps, 0.910 -> 0.571 at 12, 0.430 -> 0.308 at 8.
 #pragma once
 
 #include "grid2d_kernels.cuh"
@@ -24,9 +27,9 @@ constexpr int kOneMaxW = 14;  // W / 2 + 1 lanes a row, at most 8
 
 // Bins of at most this many samples read their taps from the grid itself (through L1) instead
 // of staging a window: a window is 5,000 to 6,900 cells however few the samples.  Measured
-// against staging every bin: 256,000 samples of 12 taps on a 192^3 grid (35 a bin) 0.41 ->
-// 0.38 ms; 768,000 of 10 taps (110 a bin) unchanged at 0.39 ms; reading all bins directly
-// takes 0.40 and 0.58 ms.
+// against staging every bin: 256,000 samples of 12 taps on a 192^3 grid (35 a bin) 0.285 ->
+// 0.262 ms; 115,000 of 10 taps (15 a bin) 0.132 -> 0.108; 768,000 of 10 taps (110 a bin) 0.378
+// -> 0.372.  16 instead of 32 measures the same.
 constexpr int kOneDirect = 32;
 
 // 16-byte units per staged row
@@ -86,7 +89,7 @@ __global__ void __launch_bounds__(256) k_interp3d_one(InterpArgs a, int vec) {
     constexpr bool SIX = WT == 10;                      // 5 rows of 6 lanes; else 4 rows of 8
     constexpr int STEPS = SIX ? 2 : (WT ? (WT + 3) / 4 : (kOneMaxW + 3) / 4);
     const int grow = SIX ? lane / 6 : lane >> 3, pz = SIX ? lane % 6 : lane & 7;
-    const int row0 = SIX ? (grow == 4 ? 8 : (grow == 0 ? 0 : 8 - 2 * grow)) : grow;  // {0, 6, 4, 2, 8}
+    const int row0 = SIX ? (grow >= 4 ? 8 : (grow == 0 ? 0 : 8 - 2 * grow)) : grow;  // {0, 6, 4, 2, 8}
     const bool live = SIX ? lane < 30 : pz <= W / 2;
     const int rstep = SIX ? 1 : 4;
     const int kk = lane & 15;
@@ -133,7 +136,8 @@ __global__ void __launch_bounds__(256) k_interp3d_one(InterpArgs a, int vec) {
             const float v = __shfl_sync(0xffffffffu, myw, 16 + min(ky, 15));
             wy[i] = live && ky < W ? v : 0.f;
         }
-        // a lane without taps repeats the sample's first pair (its sums are not used)
+        // a lane without taps repeats its row's first pair (its sums are not used), which a lane of
+        // its quarter warp reads anyway: any other pair would be a bank conflict
         int off[STEPS];
         float2 a0 = make_float2(0.f, 0.f), a1 = make_float2(0.f, 0.f);
         auto plane_sum = [&](const float4 *plane, float wx) {
@@ -151,7 +155,7 @@ __global__ void __launch_bounds__(256) k_interp3d_one(InterpArgs a, int vec) {
             const int y0 = ws1 + rel[1], gz = wrap_fast(zs + (zr & ~1) + (live ? 2 * pz : 0), nf2) >> 1;
 #pragma unroll
             for (int i = 0; i < STEPS; ++i)
-                off[i] = wrap_fast(y0 + (live ? row0 + rstep * i : 0), nf1) * (nf2 >> 1) + gz;
+                off[i] = wrap_fast(y0 + row0 + rstep * i, nf1) * (nf2 >> 1) + gz;
             const float4 *gb = reinterpret_cast<const float4 *>(gbase);
             const int64_t ps = (int64_t)nf1 * (nf2 >> 1);
             int gx = wrap_fast(ws0 + rel[0], nf0);
@@ -163,7 +167,7 @@ __global__ void __launch_bounds__(256) k_interp3d_one(InterpArgs a, int vec) {
         } else {
             const float4 *base = smem_i1 + ((size_t)rel[0] * WY + rel[1]) * R + (zr >> 1);
 #pragma unroll
-            for (int i = 0; i < STEPS; ++i) off[i] = live ? (row0 + rstep * i) * R + pz : 0;
+            for (int i = 0; i < STEPS; ++i) off[i] = (row0 + rstep * i) * R + (live ? pz : 0);
 #pragma unroll(WT ? WT : 2)
             for (int kx = 0; kx < W; ++kx)
                 plane_sum(base + (size_t)kx * WY * R, __shfl_sync(0xffffffffu, myw, kx));

@@ -13,8 +13,8 @@
 // the plane stride being 4 (mod 8).
 //
 // 20 density iterations (spread and interp), k_interp3d_one -> this kernel: 768,000 samples on a
-// 192^3 grid, 10 taps 15.11 -> 13.83 ms, 8 taps 15.67 -> 9.73 ms; 2,560,000 samples on 256^3, 10
-// taps 45.4 -> 41.3 ms; 192,000 on 192^3, 12 taps 8.39 -> 5.27 ms.  64 registers for four
+// 192^3 grid, 10 taps 14.83 -> 13.81 ms, 8 taps 11.67 -> 9.73 ms; 2,560,000 samples on 256^3, 10
+// taps 44.6 -> 41.3 ms; 192,000 on 128^3, 12 taps 6.28 -> 5.30 ms.  64 registers for four
 // blocks an SM (74 and three blocks without the bound: 14.06 ms in the first case).
 #pragma once
 
