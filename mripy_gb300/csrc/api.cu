@@ -413,8 +413,11 @@ int interp_cg(const gbn_plan *p) {
     int n_pow2 = 1;
     while (n_pow2 < n) n_pow2 *= 2;
     if (cg > n_pow2) cg = n_pow2;
-    // 3-D, up to 3 coils: a block per coil
-    if (cg <= 0 && p->dim == 3 && n <= 3 && interp3d_one_applies(p->gi)) cg = 1;
+    // 3-D, up to 6 coils off the tensor cores: a block per coil.  Measured at 10 taps against
+    // groups of 4 or 8 on the plane-streaming kernel: 192,000 samples on 128^3, 4, 5, 6, 7 coils
+    // 487 -> 384, 696 -> 473, 701 -> 564, 706 -> 654 us; 768,000 on 192^3, 4 and 6 coils 1689 ->
+    // 1407, 2401 -> 2098; 12 taps, 192,000 samples, 4, 6, 7 coils 655 -> 589, 978 -> 881, 982 -> 1022
+    if (cg <= 0 && p->dim == 3 && n <= 6 && interp3d_one_applies(p->gi)) cg = 1;
     if (cg <= 0) {
         int best = 1 << 30;
         for (int cand : {8, 4, 2, 1}) {

@@ -170,3 +170,30 @@ def test_one_coil_interp_samples_in_every_cell_of_a_bin(eps, ns):
     G = cvec(rng, (1,) + nf)
     assert rel(p.interp(cuda(G)), np.prod(nf) * O.interp(tuple(xs), G, tau, nsp).T) < TOL_REF
     p.close()
+
+
+@pytest.mark.parametrize("nc", [4, 5, 6])
+@pytest.mark.parametrize("shape,eps", [((26, 25, 24), 1e-5), ((19, 18, 17), 1e-12), ((24, 24, 24), 5e-6), ((22, 20, 24), 1e-3)])
+def test_four_to_six_coils_interp_against_oracle(nc, shape, eps):
+    """These run one coil per block too: staged and sparse bins, two groups, odd grids, coil-major
+    samples, and the caller's own coil group agrees."""
+    rng = np.random.default_rng(nc)
+    off = [0, 3000, 9000]
+    M = off[-1]
+    xs = _points(rng, M)
+    p = NufftPlan(3, shape, n_coil=nc, n_traj=2, eps=eps, max_nspread=6)
+    p.set_points([cuda(v) for v in xs], traj_offsets=off)
+    nsp, nf, tau = O.grid_params(3, *shape, eps=eps, max_nspread=6)
+    assert p.info()["interp_coil_group"] == 1
+    G = cvec(rng, (2, nc) + nf)
+    km = torch.empty((nc, M), dtype=torch.complex64, device="cuda").t()
+    k = p.interp(cuda(G), out=km).cpu().numpy()
+    for g in (0, 1):
+        sl = slice(off[g], off[g + 1])
+        ref = np.prod(nf) * O.interp(tuple(v[sl] for v in xs), G[g], tau, nsp).T
+        assert rel(k[sl], ref) < TOL_REF
+    q = NufftPlan(3, shape, n_coil=nc, n_traj=2, eps=eps, max_nspread=6, tuning=Tuning(interp_coil_group=4))
+    q.set_points([cuda(v) for v in xs], traj_offsets=off)
+    assert rel(q.interp(cuda(G)), k) < 2e-6
+    p.close()
+    q.close()
