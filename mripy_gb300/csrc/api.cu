@@ -617,8 +617,9 @@ int set_points_impl(gbn_plan *p, int dtype, const void *x, const void *y, const 
 
     TileTotals *totals = p->counts.as<TileTotals>();
     uint32_t *home_count = (uint32_t *)(totals + 1), *scount = home_count + Ti;
+    std::vector<float> gscale;  // read by a queued copy: alive until the synchronisation below
     if (nt > 1 || M == 0) {
-        std::vector<float> gscale(nt);
+        gscale.resize(nt);
         for (int g = 0; g < nt; ++g) {
             const int64_t Mg = off[g + 1] - off[g];
             gscale[g] = Mg > 0 ? (float)(1.0 / (double)Mg) : 0.f;
