@@ -215,6 +215,7 @@ void few_tile(int n_coil, int tile[3]);
 // the wide-stencil 2-D kernels (spread2d_wide.cuh on 32 x 32 tiles, interp2d_wide.cuh) take this
 // geometry
 constexpr int kWideMinW = 18, kWideMaxW = 30;  // taps per axis
+constexpr int kMaxGridY = 65535;  // blocks along y; these kernels take more coils in several launches
 bool spread_wide_applies(const Geom &g);
 bool interp_wide_applies(const Geom &g);
 // kernels launch_spread runs for these arguments (the 3-D register path adds a Kahan instance)

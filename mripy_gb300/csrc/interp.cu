@@ -107,8 +107,12 @@ cudaError_t launch_interp(const InterpArgs &a, int64_t n_sub, int coil_group, in
         const int vec = (uintptr_t)a.grid % 16 == 0 && a.g.nf[1] % 2 == 0 && a.g.G % 2 == 0;
         err = set_smem(k_interp2d_wide, smem);
         if (err != cudaSuccess) return err;
-        k_interp2d_wide<<<dim3((unsigned)n_sub, (unsigned)a.g.n_coil), threads > 256 ? 256 : threads, smem, s>>>(a, vec);
-        return cudaGetLastError();
+        for (int c0 = 0; c0 < a.g.n_coil && err == cudaSuccess; c0 += kMaxGridY) {
+            const dim3 blocks((unsigned)n_sub, (unsigned)std::min(a.g.n_coil - c0, kMaxGridY));
+            k_interp2d_wide<<<blocks, threads > 256 ? 256 : threads, smem, s>>>(a, vec, c0);
+            err = cudaGetLastError();
+        }
+        return err;
     }
     if (a.g.dim == 3 && a.g.W <= 16) {
         const int th = threads > 256 ? 256 : threads;

@@ -24,11 +24,11 @@ inline size_t interp2d_wide_smem(const Geom &g) {
     return ((size_t)(g.tile[0] + g.W - 1) * wide_row_units(g) + 1) * sizeof(float4);
 }
 
-__global__ void __launch_bounds__(256) k_interp2d_wide(InterpArgs a, int vec) {
+__global__ void __launch_bounds__(256) k_interp2d_wide(InterpArgs a, int vec, int coil0) {
     extern __shared__ float4 smem_iw[];  // [WX][R] pairs of y cells
     const Geom &g = a.g;
     const int4 sub = a.subs[blockIdx.x];
-    const int coil = blockIdx.y, grp = sub.x / g.ntiles;
+    const int coil = coil0 + blockIdx.y, grp = sub.x / g.ntiles;
     int o[3], e[3];
     tile_coords<2>(g, sub.x % g.ntiles, o, e);
     const int W = g.W, ns = g.ns;

@@ -103,6 +103,7 @@ int spread_path_kind(const Geom &g, int coil_group, int variant, int threads) {
 
 int spread_kernel_count(const SpreadArgs &a, int64_t n_sub, int coil_group, int threads) {
     if (n_sub == 0) return 0;
+    if (spread_wide_applies(a.g)) return (a.g.n_coil + kMaxGridY - 1) / kMaxGridY;
     const bool two = cube_path(a.g, coil_group, a.variant) || mma_path(a.g, coil_group, a.variant) ||
                      reg3d_path(a.g, coil_group, threads);
     return (two && a.any_dense) ? 2 : 1;
@@ -180,8 +181,12 @@ cudaError_t launch_spread(const SpreadArgs &a, int64_t n_sub, int coil_group, in
         return err;
     }
     if (spread_wide_applies(a.g)) {
-        k_spread2d_wide<<<dim3((unsigned)n_sub, (unsigned)a.g.n_coil), kWideWarps * 32, kWideSmem, s>>>(a);
-        return cudaGetLastError();
+        for (int c0 = 0; c0 < a.g.n_coil && err == cudaSuccess; c0 += kMaxGridY) {
+            const dim3 blocks((unsigned)n_sub, (unsigned)std::min(a.g.n_coil - c0, kMaxGridY));
+            k_spread2d_wide<<<blocks, kWideWarps * 32, kWideSmem, s>>>(a, c0);
+            err = cudaGetLastError();
+        }
+        return err;
     }
     // few-coil 3-D kernel
     if (few_applies(a.g)) {

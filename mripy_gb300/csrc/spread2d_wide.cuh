@@ -23,11 +23,11 @@ constexpr int kWideTile = 32, kWideWarps = 4, kWideStride = 68;  // floats per s
 constexpr size_t kWideSmem = (size_t)kWideWarps * 32 * kWideStride * sizeof(float);
 static_assert(kWideSmem >= 2 * 32 * 33 * sizeof(float2), "two partial tiles");
 
-__global__ void __launch_bounds__(kWideWarps * 32, 4) k_spread2d_wide(SpreadArgs a) {
+__global__ void __launch_bounds__(kWideWarps * 32, 4) k_spread2d_wide(SpreadArgs a, int coil0) {
     extern __shared__ float4 smem_wide[];
     const Geom &g = a.g;
     const int4 sub = a.subs[blockIdx.x];
-    const int coil = blockIdx.y, grp = sub.x / g.ntiles;
+    const int coil = coil0 + blockIdx.y, grp = sub.x / g.ntiles;
     int o[3], e[3];
     tile_coords<2>(g, sub.x % g.ntiles, o, e);
     // (tile_coords' axes 0, 1 of a 2-D grid)
