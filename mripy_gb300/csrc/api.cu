@@ -600,13 +600,14 @@ int set_points_impl(gbn_plan *p, int dtype, const void *x, const void *y, const 
     const int64_t Ti = (int64_t)p->gi.ntiles * nt, Ts = (int64_t)p->gs.ntiles * nt;
     // one buffer, zeroed by one memset: totals and status, counts per interp bin and spread tile
     const size_t count_bytes = sizeof(TileTotals) + sizeof(uint32_t) * (size_t)(Ti + Ts);
+    const size_t part_at = (count_bytes + 15) / 16 * 16;  // and, behind it, scratch of the scan
     GBN_TRY(ensure(p, p->traj_off_d, sizeof(int64_t) * (nt + 1)));
     GBN_TRY(ensure(p, p->grp_scale, sizeof(float) * nt));
     GBN_TRY(ensure(p, p->pts, sizeof(float4) * Mb));
     GBN_TRY(ensure(p, p->home_key, sizeof(uint32_t) * Mb));
     GBN_TRY(ensure(p, p->touch_count, sizeof(uint32_t) * Mb));
     GBN_TRY(ensure(p, p->touch_off, sizeof(uint64_t) * Mb));
-    GBN_TRY(ensure(p, p->counts, count_bytes));
+    GBN_TRY(ensure(p, p->counts, part_at + sizeof(TileSums) * 2 * kScanChunks));
     GBN_TRY(ensure(p, p->home_pts, sizeof(float4) * Mb));
     GBN_TRY(ensure(p, p->scratch, sizeof(float2) * Mb * (size_t)p->desc.n_coil));
     GBN_TRY(ensure(p, p->split_tiles, sizeof(uint32_t) * (size_t)std::max<int64_t>(Ts, 1)));
@@ -671,7 +672,7 @@ int set_points_impl(gbn_plan *p, int dtype, const void *x, const void *y, const 
     ji.sub_off = p->sub_off_i.as<uint32_t>();
     ji.T = Ti;
     ji.max_sub = interp_max_sub;
-    GBN_CUDA(launch_tile_scan(js, ji, totals, s));
+    GBN_CUDA(launch_tile_scan(js, ji, (TileSums *)((char *)p->counts.p + part_at), totals, s));
 
     uint32_t *tc = p->touch_count.as<uint32_t>();
     uint64_t *to = p->touch_off.as<uint64_t>();

@@ -139,7 +139,14 @@ struct TileTotals {  // zeroed by the caller, with the counts
     uint32_t status;               // bit 0: a coordinate is not finite
     uint32_t split_cursor, dense_cursor, pad;
 };
-cudaError_t launch_tile_scan(const SubsJob &spread, const SubsJob &home, TileTotals *out, cudaStream_t s);
+struct TileSums {
+    uint64_t entries, items;
+};
+constexpr int kScanOneBlock = 16384;  // tiles that one block scans
+constexpr int kScanChunks = 1024;     // chunks of more tiles (a chunk's base is summed a chunk a thread)
+// part: 2 * kScanChunks sums of scratch
+cudaError_t launch_tile_scan(const SubsJob &spread, const SubsJob &home, TileSums *part, TileTotals *out,
+                             cudaStream_t s);
 cudaError_t launch_build_subs(const SubsJob &spread, const SubsJob &home, cudaStream_t s);
 
 // grid.cu

@@ -182,19 +182,77 @@ __device__ __forceinline__ uint32_t items_of(uint32_t c, const SubsJob &j) {
     return j.every_tile && s == 0 ? 1u : s;
 }
 
+// sums of a block's 64-bit pairs, in thread 0 (sh: 64 words)
+__device__ __forceinline__ void block_sum(uint64_t &c, uint64_t &s, uint64_t *sh) {
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) {
+        c += __shfl_down_sync(0xffffffffu, c, m);
+        s += __shfl_down_sync(0xffffffffu, s, m);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        sh[2 * (threadIdx.x >> 5)] = c;
+        sh[2 * (threadIdx.x >> 5) + 1] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int w = 1; w < 32; ++w) {
+            c += sh[2 * w];
+            s += sh[2 * w + 1];
+        }
+}
+
+// entries and work items of each chunk of tiles, for k_tile_scan over several blocks
+__global__ void __launch_bounds__(1024) k_tile_sums(SubsJob spread, SubsJob home, int64_t chunk, TileSums *part) {
+    const SubsJob &j = blockIdx.y == 0 ? spread : home;
+    __shared__ uint64_t sh[64];
+    const int64_t t0 = blockIdx.x * chunk, t1 = min(t0 + chunk, j.T);
+    uint64_t c = 0, s = 0;
+#pragma unroll 4
+    for (int64_t t = t0 + threadIdx.x; t < t1; t += 1024) {
+        const uint32_t n = j.count[t];
+        c += n;
+        s += items_of(n, j);
+    }
+    block_sum(c, s, sh);
+    if (threadIdx.x == 0) part[blockIdx.y * gridDim.x + blockIdx.x] = TileSums{c, s};
+}
+
 // Per tile, the exclusive sums of its entries (tile_off) and of its work items (sub_off), and
-// the totals.  One block per bin geometry walks its tiles 4096 at a time (1,024 to 37,000
-// tiles in the benchmark workloads): it stands for two device scans and a count kernel per
-// geometry, whose ten launches and separate read-backs took longer than the work.
-__global__ void __launch_bounds__(1024) k_tile_scan(SubsJob spread, SubsJob home, TileTotals *out) {
-    const SubsJob &j = blockIdx.x == 0 ? spread : home;
+// the totals.  A block walks its chunk of tiles 4096 at a time.  Up to kScanOneBlock tiles one
+// block per bin geometry does it all: it stands for two device scans and a count kernel per
+// geometry, whose ten launches and separate read-backs took longer than the work.  A step is a
+// chain of loads, shuffles and two barriers, 4.5 us, so more tiles (many groups, large 3-D grids)
+// are cut into chunks, whose sums k_tile_sums leaves in `part` before.  set_points, one block ->
+// chunks (device scans): 512 frames of 128^2, 262,144 bins 553 -> 266 us (467); 4096 frames,
+// 2.1 M bins 3414 -> 1113 (1549); 384^3 image, 884,736 bins 1613 -> 645 (970).
+__global__ void __launch_bounds__(1024) k_tile_scan(SubsJob spread, SubsJob home, int64_t chunk,
+                                                    const TileSums *part, TileTotals *out) {
+    const bool is_spread = blockIdx.y == 0, last = blockIdx.x + 1 == gridDim.x;
+    const SubsJob &j = is_spread ? spread : home;
     __shared__ uint64_t sh_c[32];
     __shared__ uint32_t sh_s[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint64_t base_c = 0;
     uint64_t base_s = 0;
+    if (blockIdx.x > 0) {  // the chunks in front (at most 1024: one a thread)
+        __shared__ uint64_t sh[64], base[2];
+        if (threadIdx.x < blockIdx.x) {
+            const TileSums p = part[blockIdx.y * gridDim.x + threadIdx.x];
+            base_c = p.entries;
+            base_s = p.items;
+        }
+        block_sum(base_c, base_s, sh);
+        if (threadIdx.x == 0) {
+            base[0] = base_c;
+            base[1] = base_s;
+        }
+        __syncthreads();
+        base_c = base[0];
+        base_s = base[1];
+    }
     uint32_t dense = 0, split = 0;
-    for (int64_t t0 = 0; t0 < j.T; t0 += 4096) {
+    const int64_t end = min((blockIdx.x + 1) * chunk, j.T);
+    for (int64_t t0 = blockIdx.x * chunk; t0 < end; t0 += 4096) {
         const int64_t t = t0 + 4 * threadIdx.x;
         uint32_t c[4], s[4];
         uint64_t sum_c = 0;
@@ -249,7 +307,7 @@ __global__ void __launch_bounds__(1024) k_tile_scan(SubsJob spread, SubsJob home
         base_s += ts;
         __syncthreads();  // sh_* are read
     }
-    if (blockIdx.x == 0) {
+    if (is_spread) {
         dense = __reduce_add_sync(0xffffffffu, dense);
         split = __reduce_add_sync(0xffffffffu, split);
         if (lane == 0) {
@@ -257,9 +315,9 @@ __global__ void __launch_bounds__(1024) k_tile_scan(SubsJob spread, SubsJob home
             atomicAdd(&out->n_split, split);
         }
     }
-    if (threadIdx.x == 0) {
-        (blockIdx.x == 0 ? out->entries : out->home_entries) = base_c;
-        (blockIdx.x == 0 ? out->spread_subs : out->interp_subs) = base_s;
+    if (threadIdx.x == 0 && last) {
+        (is_spread ? out->entries : out->home_entries) = base_c;
+        (is_spread ? out->spread_subs : out->interp_subs) = base_s;
     }
 }
 
@@ -324,8 +382,18 @@ cudaError_t launch_gather_pts(const float4 *pts, const uint32_t *idx, int64_t n,
     return cudaGetLastError();
 }
 
-cudaError_t launch_tile_scan(const SubsJob &spread, const SubsJob &home, TileTotals *out, cudaStream_t s) {
-    k_tile_scan<<<2, 1024, 0, s>>>(spread, home, out);
+cudaError_t launch_tile_scan(const SubsJob &spread, const SubsJob &home, TileSums *part, TileTotals *out,
+                             cudaStream_t s) {
+    const int64_t T = spread.T > home.T ? spread.T : home.T;
+    int64_t chunk = T > 4096 ? (T + 4095) / 4096 * 4096 : 4096;
+    if (T > kScanOneBlock) chunk = (T + 4096 * (int64_t)kScanChunks - 1) / (4096 * (int64_t)kScanChunks) * 4096;
+    const dim3 blocks((unsigned)((T + chunk - 1) / chunk), 2);
+    if (blocks.x > 1) {
+        k_tile_sums<<<blocks, 1024, 0, s>>>(spread, home, chunk, part);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    k_tile_scan<<<blocks, 1024, 0, s>>>(spread, home, chunk, part, out);
     return cudaGetLastError();
 }
 
