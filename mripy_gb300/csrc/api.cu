@@ -83,6 +83,7 @@ struct gbn_plan {
     Geom gs{}, gi{};
     int coil_group = 1, threads = 256, interp_threads = 256, max_sub = 256, interp_coil_group = 0;
     int interp_max_sub = 1 << 30;  // interp work items where the spread's own size is longer
+    bool auto_bins = false;  // 2-D: set_points chooses the interp bins (interp_bins2d)
     int interp_staging = 0;  // 0: tensor copies where the grid allows, 1: thread loads
     int interp_variant = 0;  // 3-D, 8 coils: 0 library choice, 1 interp bins, 2 tensor cores
     int spread_variant = 0;  // 3-D, 8 coils: 0 library choice, 1 warp rows, 2 cubes, 3 tensor cores
@@ -432,6 +433,30 @@ int interp_cg(const gbn_plan *p) {
     return cg;
 }
 
+// The interp bins of a 2-D plan whose caller chose none, by taps, coils per block and samples.
+// 8 x 16 bins stage windows small enough for more blocks per SM, or more coils an item, than
+// 16 x 16 ones, but halve the samples that share a window and a block's warps.  Which one gains was
+// measured on 561 plans (32^2 to 512^2, 1 to 20 frames, radial, spiral and random samples), as the
+// time with 8 x 16 bins over that with 16 x 16, geometric means: 8 coils a block 12 taps 0.94, 14
+// 0.97, 16 0.77, 4 to 10 taps 1.08, but 0.93 from 56 samples per 8 x 16 cells; 4 coils a block 8
+// to 12 taps 0.90, 4 and 6 1.09, 14 and 16 1.22; 2 coils 1.04, 1 coil 1.10; any of them with few
+// bins (up to 224 of 16 x 16), which leave the GPU idle, 0.96.  12 coils, 64 frames of 192^2, 10
+// taps: 792 -> 587 us; 2 coils, 20 frames of 256^2, 12 taps: 89 against 144 us.  Over all of them
+// the rule's choice takes 0.96 of the time of either.
+// The wide-stencil kernel (18 to 30 taps) has 8 x 16 bins, wider stencils 16 x 16.
+void interp_bins2d(gbn_plan *p) {
+    const int W = 2 * p->ns, cg = interp_cg(p);
+    const int64_t items = (int64_t)((p->nf[0] + 15) / 16) * ((p->nf[1] + 15) / 16) * p->desc.n_traj *
+                          ((p->desc.n_coil + cg - 1) / cg);
+    bool half;
+    if (W > 16) half = W <= kWideMaxW;
+    else if (items <= 224) half = true;
+    else if (cg >= 8) half = W >= 12 || 128.0 * (double)p->M >= 56.0 * p->nf[0] * p->nf[1] * p->desc.n_traj;
+    else half = cg >= 4 && W >= 8 && W <= 12;
+    const int tile[3] = {half ? 8 : 16, 16, 1};
+    make_geom(p, tile, p->gi);
+}
+
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link against the
 // driver library); null when the driver does not provide it
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
@@ -595,6 +620,7 @@ int set_points_impl(gbn_plan *p, int dtype, const void *x, const void *y, const 
     p->points_set = false;
     p->M = M;
     p->traj_off.assign(off, off + nt + 1);
+    if (p->auto_bins) interp_bins2d(p);
 
     const size_t Mb = (size_t)std::max<int64_t>(M, 1);
     const int64_t Ti = (int64_t)p->gi.ntiles * nt, Ts = (int64_t)p->gs.ntiles * nt;
@@ -894,12 +920,9 @@ int plan_create_impl(const gbn_plan_desc *desc, gbn_plan **out) {
         dspread[0] = 1024; dinterp[0] = 1024;
     } else if (p->dim == 2) {
         // measured on GB300 for the 8-coil 512^2 radial workload: 16x32 output tiles keep
-        // four spread blocks resident per SM; 8x16 interp bins keep the staged windows small
-        // enough for a ring of three or four (against 16x16 bins: 12 coils, 64 frames of 192^2
-        // 0.79 -> 0.63 ms; 8 coils of 256^2 101 -> 95 us; 16 coils 199 -> 182 us, spiral 66 ->
-        // 57 us; 6 coils and 20 frames of 128^2 2 % slower)
+        // four spread blocks resident per SM; interp bins: interp_bins2d
         dspread[0] = 16; dspread[1] = 32;
-        dinterp[0] = 8; dinterp[1] = 16;
+        dinterp[0] = dinterp[1] = 16;
     } else {
         // warp lanes run along z: 32-cell z rows for the spread tile, 8^3 interp bins
         dspread[0] = 8; dspread[1] = 8; dspread[2] = 32;
@@ -1039,6 +1062,8 @@ int plan_create_impl(const gbn_plan_desc *desc, gbn_plan **out) {
         delete p;
         return fail(GBN_ERR_CUDA, std::string("no CUDA device: ") + cudaGetErrorString(e));
     }
+    p->auto_bins = p->dim == 2 && desc->interp_tile[0] <= 0 && desc->interp_tile[1] <= 0;
+    if (p->auto_bins) interp_bins2d(p);
 
     auto bail = [&](int code) {
         gbn_plan_destroy(p);
@@ -1367,7 +1392,15 @@ int gbn_interp_grad_coords(gbn_plan *p, const void *grid, const void *grad_c, gb
     a.out = grad_xyz;
     a.scale = (float)p->desc.df;
     const int cg = interp_cg(p);
-    GBN_CUDA(launch_interp_grad(a, p->n_interp_sub, cg, p->interp_threads, s));
+    // Many 8 x 16 bins chosen by the plan: blocks of 256 threads, so that a block's warps find as
+    // many samples each as in 16 x 16 bins.  Against those (420 plans): from 1024 blocks on 1.11 to
+    // 1.20 times the time with 512 threads, 0.95 to 1.05 with 256; fewer blocks, which all fit the
+    // GPU at once, 0.95 with 512 and 1.05 with 256.
+    int threads = p->interp_threads;
+    if (p->auto_bins && p->desc.interp_threads <= 0 && p->gi.tile[0] < std::min(16, p->nf[0]) &&
+        p->n_interp_sub * ((p->desc.n_coil + cg - 1) / cg) >= 1024)
+        threads = 256;
+    GBN_CUDA(launch_interp_grad(a, p->n_interp_sub, cg, threads, s));
     return GBN_OK;
 }
 
