@@ -528,7 +528,6 @@ __global__ void __launch_bounds__(512) k_interp_grad2d(GradArgs a, float dsc0, f
         const float2 *base = a.grid + ((int64_t)grp * g.n_coil + cg0) * g.G;
         const int nitem = WX * WY * CG;
         const float rWY = 1.f / (float)WY;
-#pragma unroll 8
         for (int i = threadIdx.x; i < nitem; i += blockDim.x) {
             const int c = i % CG, cell = i / CG;
             const int wx = div_small(cell, rWY), wy = cell - wx * WY;
@@ -543,23 +542,9 @@ __global__ void __launch_bounds__(512) k_interp_grad2d(GradArgs a, float dsc0, f
     const int kk = lane & 15;
     const float beta = lane < 16 ? g.beta2[0] : g.beta2[1];
     const float dsc = lane < 16 ? dsc0 : dsc1;
-    // records one sample ahead, a sample's upstream gradient before its taps: neither load is
-    // waited for where it is used
-    float4 p_next = make_float4(0.f, 0.f, 0.f, 0.f);
-    uint32_t j_next = 0;
-    if (warp < sub.z) {
-        p_next = a.pts[(int64_t)sub.y + warp];
-        j_next = a.idx[(int64_t)sub.y + warp];
-    }
     for (int s = warp; s < sub.z; s += nw) {
-        const float4 p = p_next;
-        const uint32_t j = j_next;
-        float2 up = make_float2(0.f, 0.f);
-        if (q == 0 && cg0 + c < g.n_coil) up = a.gc[(int64_t)j * a.c_elem + (int64_t)(cg0 + c) * a.c_coil];
-        if (s + nw < sub.z) {
-            p_next = a.pts[(int64_t)sub.y + s + nw];
-            j_next = a.idx[(int64_t)sub.y + s + nw];
-        }
+        const float4 p = a.pts[(int64_t)sub.y + s];
+        const uint32_t j = a.idx[(int64_t)sub.y + s];
         int c0x, c0y, c0z;
         unpack_cells(2, __float_as_uint(p.w), c0x, c0y, c0z);
         int ccx = c0x + ns - 1, ccy = c0y + ns - 1;
@@ -622,8 +607,9 @@ __global__ void __launch_bounds__(512) k_interp_grad2d(GradArgs a, float dsc0, f
         // Re(conj(gc) * dc/dx) per coil (slot-0 lanes), then summed over the coils
         float g0 = 0.f, g1 = 0.f;
         if (q == 0 && cg0 + c < g.n_coil) {
-            g0 = up.x * gx_re + up.y * gx_im;
-            g1 = up.x * gy_re + up.y * gy_im;
+            const float2 gc = a.gc[(int64_t)j * a.c_elem + (int64_t)(cg0 + c) * a.c_coil];
+            g0 = gc.x * gx_re + gc.y * gx_im;
+            g1 = gc.x * gy_re + gc.y * gy_im;
         }
 #pragma unroll
         for (int off = 1; off < CG; off <<= 1) {
