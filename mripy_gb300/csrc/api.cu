@@ -403,9 +403,34 @@ int run_spread(gbn_plan *p, const void *c, gbn_layout L, const float *weight, fl
     return GBN_OK;
 }
 
-// Interp coils per block: the caller's choice, else the group size that pads the coil
-// count least (every padded lane still reads the window), counting 2 lanes of fixed cost
-// per block: 12 coils -> 3 groups of 4, 8 -> 1 of 8, 5 -> 1 of 8, 3 -> 1 of 4.
+// 3-D interps off the tensor cores: whether a block per coil (interp3d_one.cuh) is faster than
+// groups of 2 (k_interp3d), 4 or 8 coils (the plane-streaming kernel).  It is from 8 taps up to 3
+// coils, and for 4 to 6 coils while the bins are few (more blocks) or hold many samples: below
+// that a bin's samples read their taps from the grid, which in large grids no longer come from
+// L1.  Few taps leave most of its lanes idle.  Measured on 320 plans (1 to 7 coils, 40^3 to 192^3
+// grids, 1 to 250 samples a bin, radial and random), groups -> a block per coil: 4 taps, 6 coils,
+// 361,000 samples on 128^3 365 -> 810 us, 2,400 on 40^3 25 -> 17; 6 taps, 4 coils, 108,000 on
+// 128^3 165 -> 205, 2,800 on 96^3 41 -> 25; 8 taps, 4 coils, 131,000 on 192^3 392 -> 706, 172,000
+// on 128^3 342 -> 296; 10 taps, 4 coils, 192,000 on 128^3 487 -> 384; 12 taps, 4 coils, 29,500 on
+// 192^3 385 -> 601, 5 coils, 192,000 on 192^3 1078 -> 985; 14 taps, 6 coils, 201,000 on 192^3
+// 1880 -> 3747, 145,000 on 96^3 1200 -> 1114.
+bool interp_one_coil(const gbn_plan *p) {
+    if (p->dim != 3 || !interp3d_one_applies(p->gi)) return false;
+    const int W = p->gi.W;
+    const int64_t n = p->desc.n_coil, M = p->M, T = (int64_t)p->gi.ntiles * p->gi.n_traj;
+    if (W <= 4) return n * M <= 32768 || (n <= 2 && M <= 8 * T);
+    if (W <= 6) return n == 1 || n * M <= 262144;
+    if (n <= 3) return true;
+    if (W <= 8) return T <= 4096;
+    if (W <= 10) return T <= 4096 || M >= 2 * T;
+    if (W <= 12) return T <= 4096 || M >= 8 * T;
+    return T < 4096 || (n >= 5 && M >= 64 * T);
+}
+
+// Interp coils per block: the caller's choice, else in 3-D one where that is faster
+// (interp_one_coil), else the group size that pads the coil count least (every padded lane still
+// reads the window), counting 2 lanes of fixed cost per block: 12 coils -> 3 groups of 4, 8 -> 1
+// of 8, 5 -> 1 of 8, 3 -> 1 of 4.
 int interp_cg(const gbn_plan *p) {
     const int n = std::max(1, (int)p->desc.n_coil);
     int cg = p->interp_coil_group;
@@ -414,11 +439,7 @@ int interp_cg(const gbn_plan *p) {
     int n_pow2 = 1;
     while (n_pow2 < n) n_pow2 *= 2;
     if (cg > n_pow2) cg = n_pow2;
-    // 3-D, up to 6 coils off the tensor cores: a block per coil.  Measured at 10 taps against
-    // groups of 4 or 8 on the plane-streaming kernel: 192,000 samples on 128^3, 4, 5, 6, 7 coils
-    // 487 -> 384, 696 -> 473, 701 -> 564, 706 -> 654 us; 768,000 on 192^3, 4 and 6 coils 1689 ->
-    // 1407, 2401 -> 2098; 12 taps, 192,000 samples, 4, 6, 7 coils 655 -> 589, 978 -> 881, 982 -> 1022
-    if (cg <= 0 && p->dim == 3 && n <= 6 && interp3d_one_applies(p->gi)) cg = 1;
+    if (cg <= 0 && n <= 6 && interp_one_coil(p)) cg = 1;
     if (cg <= 0) {
         int best = 1 << 30;
         for (int cand : {8, 4, 2, 1}) {
@@ -564,6 +585,7 @@ int run_interp(gbn_plan *p, const float2 *grid, void *c, gbn_layout L, const flo
     a.c_coil = L.coil_stride;
     a.weight = weight;
     a.real = real && p->M >= kRealMinBin * p->n_interp_sub ? 1 : 0;
+    a.paired = p->desc.n_coil > 1 || interp_one_coil(p) ? 1 : 0;
     const int cg = interp_cg(p);
     // 2-D: windows staged by tensor copies when the grid admits a tensor map
     TmaWin t{};

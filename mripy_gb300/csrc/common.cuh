@@ -178,6 +178,7 @@ struct InterpArgs {
     int64_t c_elem, c_coil;
     const float *weight;      // per sample (original index) or null
     int real = 0;             // the grid's imaginary parts are zero (density compensation)
+    int paired = 1;           // 3-D, one coil per block: the paired-cell kernel
 };
 struct GradArgs {
     Geom g;

@@ -118,7 +118,7 @@ cudaError_t launch_interp(const InterpArgs &a, int64_t n_sub, int coil_group, in
         const int th = threads > 256 ? 256 : threads;
         if (interp3d_planes_smem_bytes(a.g, coil_group, th))  // 4 or 8 coils: stream plane by plane
             return launch_interp3d_planes(a, n_sub, coil_group, th, nullptr, nullptr, s);
-        if (coil_group == 1 && interp3d_one_applies(a.g)) {
+        if (coil_group == 1 && a.paired && interp3d_one_applies(a.g)) {
             const int vec = (uintptr_t)a.grid % 16 == 0 && a.g.nf[2] % 2 == 0 && a.g.G % 2 == 0;
             const size_t rsmem = interp3d_real_smem_bytes(a.g);
             if (a.real && vec && rsmem > 0 && rsmem <= 112 * 1024) {
