@@ -454,6 +454,18 @@ int interp_cg(const gbn_plan *p) {
     return cg;
 }
 
+// Coils per block of the coordinate gradients: in 2-D the interp's; in 3-D (a window of all taps
+// in shared memory, one thread a sample) the caller's choice, else one for up to 6 coils (3 and 4
+// coils 0.3 to 1.0 times the time of groups of 4, 5 and 6 do not fit in groups of 8), but two for
+// 2 coils with up to 8 taps and 64 samples a bin: 119,000 samples of 8 taps on a 64^3 grid 179 ->
+// 136 us, 672,000 of 6 taps on 128^3 345 -> 290; with 10 taps one is 0.7 to 0.97 times the time.
+int grad_cg(const gbn_plan *p) {
+    const int n = p->desc.n_coil;
+    if (p->dim != 3 || p->interp_coil_group > 0 || n > 6) return interp_cg(p);
+    if (n == 2 && p->gi.W <= 8 && p->M >= 64 * (int64_t)p->gi.ntiles * p->gi.n_traj) return 2;
+    return 1;
+}
+
 // The interp bins of a 2-D plan whose caller chose none, by taps, coils per block and samples.
 // 8 x 16 bins stage windows small enough for more blocks per SM, or more coils an item, than
 // 16 x 16 ones, but halve the samples that share a window and a block's warps.  Which one gains was
@@ -1413,7 +1425,7 @@ int gbn_interp_grad_coords(gbn_plan *p, const void *grid, const void *grad_c, gb
     a.c_coil = cl.coil_stride;
     a.out = grad_xyz;
     a.scale = (float)p->desc.df;
-    const int cg = interp_cg(p);
+    const int cg = grad_cg(p);
     // Many 8 x 16 bins chosen by the plan: blocks of 256 threads, so that a block's warps find as
     // many samples each as in 16 x 16 bins.  Against those (420 plans): from 1024 blocks on 1.11 to
     // 1.20 times the time with 512 threads, 0.95 to 1.05 with 256; fewer blocks, which all fit the

@@ -46,3 +46,21 @@ def test_interp_groups(W, nc, n, M, nt, cg):
         ref = np.prod(nf) * O.interp(tuple(v[take] for v in xs), g[q * nc:(q + 1) * nc].cpu().numpy(), tau, nsp).T
         assert rel(k[take], ref) < 2e-5
     p.close()
+
+
+@pytest.mark.parametrize("W,nc,M", [(8, 2, 8000), (8, 2, 9000), (6, 2, 9000), (10, 2, 9000), (12, 4, 3000), (8, 1, 9000),
+                                    (6, 3, 3000)])
+def test_gradient_groups(W, nc, M):
+    rng = np.random.default_rng(W * nc)
+    shape = (20, 20, 20)
+    xs = [torch.from_numpy(v).cuda() for v in rng.uniform(-np.pi, np.pi, (3, M))]
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    y = torch.randn(M, nc, generator=gen, dtype=torch.complex64, device="cuda")
+    out = []
+    for cg in (0, 1, 2):
+        p = NufftPlan(3, shape, n_coil=nc, eps=EPS[W], tuning=Tuning(interp_coil_group=cg)).set_points(xs)
+        g = torch.randn(p.grid().shape, generator=torch.Generator(device="cuda").manual_seed(2), dtype=torch.complex64,
+                        device="cuda")
+        out.append(p.interp_grad_coords(g, y).cpu().numpy())
+        p.close()
+    assert rel(out[0], out[1]) < 1e-5 and rel(out[0], out[2]) < 1e-5
