@@ -405,26 +405,27 @@ int run_spread(gbn_plan *p, const void *c, gbn_layout L, const float *weight, fl
 
 // 3-D interps off the tensor cores: whether a block per coil (interp3d_one.cuh) is faster than
 // groups of 2 (k_interp3d), 4 or 8 coils (the plane-streaming kernel).  It is from 8 taps up to 3
-// coils, and for 4 to 6 coils while the bins are few (more blocks) or hold many samples: below
-// that a bin's samples read their taps from the grid, which in large grids no longer come from
-// L1.  Few taps leave most of its lanes idle.  Measured on 320 plans (1 to 7 coils, 40^3 to 192^3
-// grids, 1 to 250 samples a bin, radial and random), groups -> a block per coil: 4 taps, 6 coils,
-// 361,000 samples on 128^3 365 -> 810 us, 2,400 on 40^3 25 -> 17; 6 taps, 4 coils, 108,000 on
-// 128^3 165 -> 205, 2,800 on 96^3 41 -> 25; 8 taps, 4 coils, 131,000 on 192^3 392 -> 706, 172,000
-// on 128^3 342 -> 296; 10 taps, 4 coils, 192,000 on 128^3 487 -> 384; 12 taps, 4 coils, 29,500 on
-// 192^3 385 -> 601, 5 coils, 192,000 on 192^3 1078 -> 985; 14 taps, 6 coils, 201,000 on 192^3
-// 1880 -> 3747, 145,000 on 96^3 1200 -> 1114.
+// coils; for 4 to 6 coils with few work items, which leave the GPU idle in groups, in grids of
+// at most 4096 bins, or with many samples a bin: below that a bin's samples read their taps from
+// the grid itself, which in large grids no longer come from L1 (10 taps, whose lanes are all
+// used, are the faster all the same).  Few taps leave most of its lanes idle.  Measured on 470
+// plans (1 to 7 coils, 40^3 to 192^3 grids, 1 to 250 samples a bin, radial and random), groups ->
+// a block per coil: 4 taps, 6 coils, 361,000 samples on 128^3 365 -> 810 us, 2,400 on 40^3 25 -> 17;
+// 6 taps, 4 coils, 108,000 on 128^3 165 -> 205, 2,800 on 96^3 41 -> 25; 8 taps, 4 coils, 131,000
+// on 192^3 392 -> 706, 7,800 radial in three 96^3 76 -> 40; 10 taps, 4 coils, 192,000 on 128^3 487
+// -> 384; 12 taps, 4 coils, 29,500 on 192^3 385 -> 601, 9,500 radial 120 -> 89; 14 taps, 6 coils,
+// 201,000 on 192^3 1880 -> 3747, 436,000 radial on 128^3 3356 -> 3109.
 bool interp_one_coil(const gbn_plan *p) {
     if (p->dim != 3 || !interp3d_one_applies(p->gi)) return false;
     const int W = p->gi.W;
     const int64_t n = p->desc.n_coil, M = p->M, T = (int64_t)p->gi.ntiles * p->gi.n_traj;
+    const int64_t items = p->points_set ? p->n_interp_sub : std::min(T, M);  // (at most, while binning)
     if (W <= 4) return n * M <= 32768 || (n <= 2 && M <= 8 * T);
     if (W <= 6) return n == 1 || n * M <= 262144;
-    if (n <= 3) return true;
-    if (W <= 8) return T <= 4096;
-    if (W <= 10) return T <= 4096 || M >= 2 * T;
-    if (W <= 12) return T <= 4096 || M >= 8 * T;
-    return T < 4096 || (n >= 5 && M >= 64 * T);
+    if (n <= 3 || W == 10) return true;
+    if (W == 8) return T <= 4096 || items <= 1700;
+    if (W == 12) return n == 5 || T <= 4096 || items <= 2100 || M >= 8 * T;
+    return T < 4096 || items <= 1200 || (n >= 5 && M >= 64 * T);
 }
 
 // Interp coils per block: the caller's choice, else in 3-D one where that is faster
@@ -476,7 +477,8 @@ int grad_cg(const gbn_plan *p) {
 // bins (up to 224 of 16 x 16), which leave the GPU idle, 0.96.  12 coils, 64 frames of 192^2, 10
 // taps: 792 -> 587 us; 2 coils, 20 frames of 256^2, 12 taps: 89 against 144 us.  Over all of them
 // the rule's choice takes 0.96 of the time of either.
-// The wide-stencil kernel (18 to 30 taps) has 8 x 16 bins, wider stencils 16 x 16.
+// The wide-stencil kernel (18 to 30 taps) has 8 x 16 bins, wider stencils 16 x 16 (32 taps, 20,000
+// samples on 384^2: 53 us with 8 x 16, 35 with 16 x 16).
 void interp_bins2d(gbn_plan *p) {
     const int W = 2 * p->ns, cg = interp_cg(p);
     const int64_t items = (int64_t)((p->nf[0] + 15) / 16) * ((p->nf[1] + 15) / 16) * p->desc.n_traj *

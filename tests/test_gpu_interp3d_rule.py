@@ -25,7 +25,8 @@ def rel(a, b):
     (4, 6, 16, 5461, 1, 1), (4, 6, 16, 5462, 1, 8), (4, 2, 20, 17000, 1, 2), (4, 1, 16, 40000, 1, 1),
     (4, 2, 72, 40000, 1, 1), (6, 4, 16, 65536, 1, 1), (6, 4, 16, 65600, 1, 4), (6, 1, 16, 300000, 1, 1),
     (8, 4, 32, 9000, 8, 1), (8, 4, 32, 9000, 9, 4), (8, 3, 32, 9000, 9, 1), (10, 6, 32, 9216, 9, 1),
-    (10, 6, 32, 9000, 9, 8), (12, 4, 32, 36900, 9, 1), (12, 4, 32, 36000, 9, 4), (14, 5, 32, 4000, 7, 1),
+    (8, 4, 32, 1500, 9, 1), (12, 5, 32, 36000, 9, 1), (12, 4, 32, 2000, 9, 1),
+    (14, 4, 32, 1000, 8, 1), (12, 4, 32, 36900, 9, 1), (12, 4, 32, 36000, 9, 4), (14, 5, 32, 4000, 7, 1),
     (14, 5, 32, 4000, 8, 8), (14, 6, 16, 262200, 64, 1), (14, 4, 32, 4000, 8, 4), (14, 3, 32, 4000, 8, 1),
     (12, 7, 16, 3000, 1, 8)])
 def test_interp_groups(W, nc, n, M, nt, cg):
