@@ -6,8 +6,8 @@
 //
 // As k_interp3d_one: a warp per sample, 16 lanes read a row's taps two cells (16 bytes) at a
 // time from the even cell at or below the first, two rows a step; a cell outside the stencil
-// (its weight is zero) is left out by a select, so that a value that is not finite there does
-// not reach the sum.
+// is left out by a select on its tap, so that a value that is not finite there does not reach the
+// sum (and one inside does, also where the weight has flushed to zero).
 #pragma once
 
 #include "grid2d_kernels.cuh"
@@ -87,8 +87,8 @@ __global__ void __launch_bounds__(256) k_interp2d_wide(InterpArgs a, int vec, in
             a1 = __ffma2_rn(w2, make_float2(u.z, u.w), a1);
         }
         float x = 0.f, y = 0.f;
-        if (wy[0] != 0.f) { x = wy[0] * a0.x; y = wy[0] * a0.y; }
-        if (wy[1] != 0.f) { x = fmaf(wy[1], a1.x, x); y = fmaf(wy[1], a1.y, y); }
+        if (live && (unsigned)ky < (unsigned)W) { x = wy[0] * a0.x; y = wy[0] * a0.y; }
+        if (live && (unsigned)(ky + 1) < (unsigned)W) { x = fmaf(wy[1], a1.x, x); y = fmaf(wy[1], a1.y, y); }
 #pragma unroll
         for (int m = 16; m > 0; m >>= 1) {
             x += __shfl_xor_sync(0xffffffffu, x, m);

@@ -143,12 +143,12 @@ __global__ void __launch_bounds__(256, 4) k_interp3d_real(InterpArgs a) {
             a0 = __ffma2_rn(w2, make_float2(v.x, v.y), a0);
             a1 = __ffma2_rn(w2, make_float2(v.z, v.w), a1);
         }
-        // select, as in k_interp3d_one: cells outside the stencil may be anything
+        // select by tap, as in k_interp3d_one: cells outside the stencil may be anything
         float x = 0.f;
-        if (wz[0] != 0.f) x = wz[0] * a0.x;
-        if (wz[1] != 0.f) x = fmaf(wz[1], a0.y, x);
-        if (wz[2] != 0.f) x = fmaf(wz[2], a1.x, x);
-        if (wz[3] != 0.f) x = fmaf(wz[3], a1.y, x);
+        if ((unsigned)kz < (unsigned)W) x = wz[0] * a0.x;
+        if ((unsigned)(kz + 1) < (unsigned)W) x = fmaf(wz[1], a0.y, x);
+        if ((unsigned)(kz + 2) < (unsigned)W) x = fmaf(wz[2], a1.x, x);
+        if ((unsigned)(kz + 3) < (unsigned)W) x = fmaf(wz[3], a1.y, x);
 #pragma unroll
         for (int m = 16; m > 0; m >>= 1) x += __shfl_xor_sync(0xffffffffu, x, m);
         if (lane == 0) {

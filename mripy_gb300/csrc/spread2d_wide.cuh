@@ -12,7 +12,8 @@
 // covers them: 3.4 pairs per sample, against 7.2 with 16-cell tiles.  The four partial tiles
 // are added through shared memory in a fixed order.
 //
-// A value that is not finite reaches only its own stencil (guarded loop).
+// A value that is not finite reaches its own stencil and no other cells (guarded loop, by taps:
+// weights inside the stencil flush to zero where the grid's axes differ much).
 #pragma once
 
 #include "grid2d_kernels.cuh"
@@ -95,11 +96,13 @@ __global__ void __launch_bounds__(kWideWarps * 32, 4) k_spread2d_wide(SpreadArgs
             for (int s = 0; s < n; ++s) {
                 const float *w = st + s * kWideStride;
                 const float wx = w[lane], vx = w[64], vy = w[65];
+                const int sx = __shfl_sync(0xffffffffu, r[0], s), sy = __shfl_sync(0xffffffffu, r[1], s);
+                if ((unsigned)(lane - sx) >= (unsigned)W) continue;
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     const float ga = wx * w[32 + 2 * i], gb = wx * w[33 + 2 * i];
-                    if (ga != 0.f) { re[i].x = fmaf(ga, vx, re[i].x); im[i].x = fmaf(ga, vy, im[i].x); }
-                    if (gb != 0.f) { re[i].y = fmaf(gb, vx, re[i].y); im[i].y = fmaf(gb, vy, im[i].y); }
+                    if ((unsigned)(2 * i - sy) < (unsigned)W) { re[i].x = fmaf(ga, vx, re[i].x); im[i].x = fmaf(ga, vy, im[i].x); }
+                    if ((unsigned)(2 * i + 1 - sy) < (unsigned)W) { re[i].y = fmaf(gb, vx, re[i].y); im[i].y = fmaf(gb, vy, im[i].y); }
                 }
             }
             continue;

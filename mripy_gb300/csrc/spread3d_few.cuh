@@ -20,9 +20,9 @@
 //
 // REAL: the samples' imaginary parts are zero (density compensation): half the FMAs.
 //
-// A value that is not finite reaches only the cells of its own stencil, as with the kernels
-// that walk the stencil: a batch with such a sample takes the guarded loop, which skips the
-// zero weights instead of multiplying by them.
+// A value that is not finite reaches the cells of its own stencil and no others, as with the
+// kernels that walk the stencil: a batch with such a sample takes the guarded loop, which goes by
+// the taps (weights inside the stencil flush to zero where a grid's axes differ much).
 #pragma once
 
 #include "grid2d_kernels.cuh"
@@ -50,7 +50,7 @@ constexpr size_t few_smem_bytes(int nc) {
 __host__ __device__ constexpr int few_blocks(int nc, bool real) { return real ? 6 : (nc <= 2 ? 4 : 3); }
 
 // The lane's sample staged: first taps relative to the tile (signed), then the tile-plane
-// weights.  Returns r[2] (z) for the half masks.
+// weights.  Returns the first taps, 8 bits each, offset by 16 (few_tap).
 template <int WT, int TZ>
 __device__ __forceinline__ int few_stage(const Geom &g, const int o[3], const float4 &p, float4 *mine) {
     const int W = WT ? WT : g.W, ns = g.ns;
@@ -78,8 +78,9 @@ __device__ __forceinline__ int few_stage(const Geom &g, const int o[3], const fl
         }
         mine[q] = make_float4(w4[0], w4[1], w4[2], w4[3]);
     }
-    return r[2];
+    return (r[0] + 16) | (r[1] + 16) << 8 | (r[2] + 16) << 16;
 }
+__device__ __forceinline__ int few_tap(int packed, int d) { return (packed >> 8 * d & 255) - 16; }
 
 __device__ __forceinline__ void few_load_z(const float *w, float2 (&wz)[4]) {
     const float4 a = *reinterpret_cast<const float4 *>(w), b = *reinterpret_cast<const float4 *>(w + 4);
@@ -140,7 +141,8 @@ __global__ void __launch_bounds__(kFewWarps * 32, few_blocks(NC, REAL)) k_spread
     for (int base = warp * 32; base < sub.z; base += kFewWarps * 32) {
         const int n = min(32, sub.z - base);
         __syncwarp();  // the previous batch is consumed
-        const int rz = few_stage<WT, TZ>(g, o, p, reinterpret_cast<float4 *>(st + lane * ST));
+        const int taps = few_stage<WT, TZ>(g, o, p, reinterpret_cast<float4 *>(st + lane * ST));
+        const int rz = few_tap(taps, 2);
         bool fin = true;
 #pragma unroll
         for (int c = 0; c < NC; ++c)
@@ -161,20 +163,24 @@ __global__ void __launch_bounds__(kFewWarps * 32, few_blocks(NC, REAL)) k_spread
             for (int s = 0; s < n; ++s) {
                 const float *w = st + s * ST;
                 const float t[2] = {w[lx] * w[8 + 2 * yq], w[lx] * w[9 + 2 * yq]};
+                const int ts = __shfl_sync(0xffffffffu, taps, s);
+                const int sx = few_tap(ts, 0), sy = few_tap(ts, 1), sz = few_tap(ts, 2);
 #pragma unroll
                 for (int c = 0; c < NC; ++c)
 #pragma unroll
                     for (int k = 0; k < RI; ++k) {
                         const float u = w[16 + TZ + RI * c + k];
 #pragma unroll
-                        for (int r = 0; r < 2; ++r)
+                        for (int r = 0; r < 2; ++r) {
+                            const bool in = (unsigned)(lx - sx) < (unsigned)W && (unsigned)(2 * yq + r - sy) < (unsigned)W;
 #pragma unroll
                             for (int z = 0; z < ZP; ++z) {
-                                const float ga = t[r] * w[16 + 2 * z], gb = t[r] * w[17 + 2 * z];
                                 float2 &m = acc[c][k][r][z];
-                                if (ga != 0.f) m.x = fmaf(ga, u, m.x);
-                                if (gb != 0.f) m.y = fmaf(gb, u, m.y);
+                                if (in && (unsigned)(2 * z - sz) < (unsigned)W) m.x = fmaf(t[r] * w[16 + 2 * z], u, m.x);
+                                if (in && (unsigned)(2 * z + 1 - sz) < (unsigned)W)
+                                    m.y = fmaf(t[r] * w[17 + 2 * z], u, m.y);
                             }
+                        }
                     }
             }
             continue;
