@@ -660,6 +660,7 @@ int set_points_impl(gbn_plan *p, int dtype, const void *x, const void *y, const 
 
     const size_t Mb = (size_t)std::max<int64_t>(M, 1);
     const int64_t Ti = (int64_t)p->gi.ntiles * nt, Ts = (int64_t)p->gs.ntiles * nt;
+    if (Ts + Ti >= (int64_t)1 << 32) return fail(GBN_ERR_CAPACITY, "more than 2^32-1 tiles and bins");  // 32-bit sort keys
     // one buffer, zeroed by one memset: totals and status, counts per interp bin and spread tile
     const size_t count_bytes = sizeof(TileTotals) + sizeof(uint32_t) * (size_t)(Ti + Ts);
     const size_t part_at = (count_bytes + 15) / 16 * 16;  // and, behind it, scratch of the scan
