@@ -13,10 +13,16 @@
 // a thread reads the R1 cells j + r R2 straight from the image or grid, transforms them,
 // and writes them to shared memory; after one barrier it reads the R2 cells of output k,
 // multiplies them by the twiddles W_N^{k r} (a table rounded from FP64), transforms them and
-// writes the cells k + r R1 out.  A block takes kFftLines lines: adjacent cells of the inner
-// axis for the strided passes (128-byte rows), (row, coil) pairs for the row passes, where the
-// image side takes coils or pixels fastest, whichever is contiguous.  The transform in place
-// is safe because a block's lines are its own and all of them are read before the barrier.
+// writes the cells k + r R1 out.  A block of a strided pass takes fft_cols lines, adjacent cells
+// of the inner axis (16: 128-byte rows; 8 where a radix is above 18), a block of a row pass
+// kFftLines (row, coil) pairs, where the image side takes coils or pixels fastest, whichever is
+// contiguous.  The transform in place is safe because a block's lines are its own and all of them
+// are read before the barrier.
+//
+// Lengths: the products of two radices listed in band_fft_{a..f}.cu: 32 of the 42 even products of
+// 2, 3 and 5 from 64 to 768 (not 90, 250, 450, 486, 500, 540, 600, 648, 720 and 750), and 112,
+// 168, 224 and 336: one in ten of the even lengths there, the ones of the usual image sizes.  A plan
+// with one other axis takes pad kernel, library transform and crop kernel.
 //
 // Measured (before: pad or crop kernel and cuFFT, band-pruned in 3-D): 64 x 12 images of
 // 192^2 in 1.14 -> 0.53 ms and out 1.02 -> 0.51 ms (3.9 TB/s); 8 images of 128^3 in 0.96 ->
@@ -227,7 +233,9 @@ __device__ __forceinline__ void fft_second(const float2 *line, int k, const floa
 // OUT: only the band's cells are written (before a crop); else only the band's cells are read
 // and the others are zero (after a pad).
 template <int R1, int R2, bool OUT>
-__global__ void __launch_bounds__(FftLine<R1, R2, fft_cols(R1, R2)>::T, OUT ? FftLine<R1, R2, fft_cols(R1, R2)>::BLOCKS_OUT : FftLine<R1, R2, fft_cols(R1, R2)>::BLOCKS_IN)
+__global__ void __launch_bounds__(FftLine<R1, R2, fft_cols(R1, R2)>::T,
+                                  OUT ? FftLine<R1, R2, fft_cols(R1, R2)>::BLOCKS_OUT
+                                      : FftLine<R1, R2, fft_cols(R1, R2)>::BLOCKS_IN)
     k_fft_cols(float2 *__restrict__ grid, FftCols a) {
     using L = FftLine<R1, R2, fft_cols(R1, R2)>;
     extern __shared__ float2 sm_fft[];

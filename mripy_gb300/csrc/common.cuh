@@ -134,7 +134,7 @@ struct SubsJob {
     int4 *subs;
 };
 struct TileTotals {  // zeroed by the caller, with the counts
-    uint64_t entries, home_entries, spread_subs, interp_subs;
+    uint64_t entries, spread_subs, interp_subs;
     uint32_t n_dense, n_split;     // dense work items, split tiles (spread)
     uint32_t status;               // bit 0: a coordinate is not finite
     uint32_t split_cursor, dense_cursor, pad;
@@ -220,8 +220,8 @@ int spread_path_kind(const Geom &g, int coil_group, int variant, int threads);
 constexpr int kFewMaxCoils = 3;
 bool few_applies(const Geom &g);
 void few_tile(int n_coil, int tile[3]);
-// the wide-stencil 2-D kernels (spread2d_wide.cuh on 32 x 32 tiles, interp2d_wide.cuh) take this
-// geometry
+// the wide-stencil 2-D kernels (spread2d_wide.cuh on 32 x 32 tiles, also below 18 taps for 1 to 3
+// coils; interp2d_wide.cuh) take this geometry
 constexpr int kWideMinW = 18, kWideMaxW = 30;  // taps per axis
 constexpr int kMaxGridY = 65535;  // blocks along y; these kernels take more coils in several launches
 bool spread_wide_applies(const Geom &g);

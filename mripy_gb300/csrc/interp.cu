@@ -3,9 +3,11 @@
 // 2-D with at most 16 taps per dimension: k_interp2d_tma (persistent, windows staged by
 // tensor copies; the caller supplies the tensor map) or k_interp2d (one block per
 // subproblem, windows gathered by the threads).  3-D with at most 16 taps:
-// k_interp3d_one (one coil per block: plans of 1 to 3 coils), k_interp3d_planes (4 or 8 coils
-// per block, window streamed by x planes) or k_interp3d.
-// 2-D with 18 to 30 taps: k_interp2d_wide.  Otherwise (1-D, wider stencils): k_interp (one thread per sample).
+// k_interp3d_one (one coil per block: plans of up to 6 coils where it is the faster) or, for the
+// real grid of the density compensation, k_interp3d_real; k_interp3d_planes (4 or 8 coils per
+// block, window streamed by x planes) or k_interp3d.
+// 2-D with 18 to 30 taps: k_interp2d_wide.  Otherwise (1-D, wider stencils): k_interp (one
+// thread per sample).
 #include <algorithm>
 #include <cstring>
 

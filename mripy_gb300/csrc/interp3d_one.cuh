@@ -1,4 +1,5 @@
-// 3-D interp (type-2 gridding) of one coil per block: k_interp3d_one<WT>, for 1 to 3 coils.
+// 3-D interp (type-2 gridding) of one coil per block: k_interp3d_one<WT>, for plans of 1 to 6
+// coils where that measured faster than groups of coils (interp_one_coil in api.cu).
 //
 // What bounds it: shared-memory reads (8 bytes per tap; W^3 taps a sample) and, behind them,
 // issue.  With one coil the warp's lanes have to split a sample's own taps.  Here a lane reads

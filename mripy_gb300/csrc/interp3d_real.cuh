@@ -5,7 +5,8 @@
 // would read zeros in half of them.  The window is staged as real parts, so a lane reads four
 // z cells at once (16 bytes): 4 lanes cover a row's taps from the 4-cell unit that holds the
 // first, and the warp takes 8 rows a step.  The stencil's W * W rows are walked in one
-// sequence over all planes (10 taps: 13 steps instead of 20), each lane with a fixed table of its rows in a period of Q planes = P whole steps.
+// sequence over all planes (10 taps: 13 steps instead of 20), each lane with a fixed table of its
+// rows in a period of Q planes = P whole steps.
 //
 // A quarter warp reads two rows of 4 units each; they do not conflict when the rows lie 4 units
 // apart (mod 8).  R = 2 (mod 4) units a row makes that rows ky and ky + 2; where the row count

@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(1024) k_tile_scan(SubsJob spread, SubsJob home
         }
     }
     if (threadIdx.x == 0 && last) {
-        (is_spread ? out->entries : out->home_entries) = base_c;
+        if (is_spread) out->entries = base_c;
         (is_spread ? out->spread_subs : out->interp_subs) = base_s;
     }
 }

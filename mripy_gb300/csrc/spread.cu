@@ -3,11 +3,11 @@
 // 2-D / 3-D with at most 16 taps per dimension and 4 or 8 coils per block, on the tile shape
 // they are built for: k_spread2d_reg / k_spread3d_reg (accumulators in registers).
 // Other 2-D / 3-D tiles: k_spread2d / k_spread3d (warp-owned shared-memory rows, no atomics).
-// 2-D with 18 to 30 taps: k_spread2d_wide.  Otherwise (1-D, wider stencils, 3-D above 16 taps,
-// small grids): k_spread (shared-memory atomics).
-// 3-D with 1 to 3 coils: k_spread3d_few.  3-D with 8 coils per block also: k_spread_mma<3, ...> (tensor cores, 4 x 8 x 16 tiles) and
-// k_spread3d_cube (register cubes), each followed by the compensated cube instance for the
-// dense work items.
+// 2-D with 18 to 30 taps, or with 1 to 3 coils: k_spread2d_wide.  Otherwise (1-D, wider stencils,
+// 3-D above 16 taps, small grids): k_spread (shared-memory atomics).
+// 3-D with 1 to 3 coils: k_spread3d_few.  3-D with 8 coils per block also: k_spread_mma<3, ...>
+// (tensor cores, 4 x 8 x 16 tiles) and k_spread3d_cube (register cubes), each followed by its
+// compensated instance for the dense work items.
 #include "dispatch.cuh"
 #include "grid2d_kernels.cuh"
 #include "grid3d_kernels.cuh"
@@ -85,8 +85,8 @@ void few_tile(int n_coil, int tile[3]) {
 // the one-coil-per-block 2-D register spread applies: stencils too wide for the other 2-D kernels,
 // or 1 to 3 coils; its tile, a grid of at least tile + stencil cells per axis
 bool spread_wide_applies(const Geom &g) {
-    return g.dim == 2 && (g.W >= kWideMinW ? g.W <= kWideMaxW : g.n_coil <= kFewMaxCoils) && g.tile[0] == kWideTile && g.tile[1] == kWideTile &&
-           g.nf[0] >= kWideTile + g.W && g.nf[1] >= kWideTile + g.W;
+    return g.dim == 2 && (g.W >= kWideMinW ? g.W <= kWideMaxW : g.n_coil <= kFewMaxCoils) &&
+           g.tile[0] == kWideTile && g.tile[1] == kWideTile && g.nf[0] >= kWideTile + g.W && g.nf[1] >= kWideTile + g.W;
 }
 
 // the cube and tensor-core kernels read interleaved work items

@@ -1,5 +1,6 @@
 // 2-D spread (type-1 gridding) with wide stencils (18 to 30 taps per axis; 28 at the functions'
-// default accuracy eps = 1e-15): k_spread2d_wide, one coil per block.
+// default accuracy eps = 1e-15), and with narrower ones for 1 to 3 coils: k_spread2d_wide, one
+// coil per block.
 //
 // What bounds it: issue and latency.  A sample has up to 900 taps, so its 4 W^2 flops dwarf its
 // bytes; the general kernel spent them on shared-memory float atomics (277 us for 32,768
@@ -11,6 +12,11 @@
 // stencil reaches (skipped otherwise, warp-uniform).  32 cells a side because a stencil nearly
 // covers them: 3.4 pairs per sample, against 7.2 with 16-cell tiles.  The four partial tiles
 // are added through shared memory in a fixed order.
+//
+// 1 to 3 coils below 18 taps, against the shared-memory rows of k_spread2d: 1 coil, 20 frames of
+// 256^2 grids, 21,800 samples of 12 taps each 351 -> 90 us; 2 coils, 265,000 samples of 10 taps on
+// a 1024^2 grid 210 -> 100; 3 coils, 20 frames of 256^2, 14,800 each 416 -> 164; only sparse random
+// samples (15 a tile, 2 coils, 20 frames of 512^2) 79 -> 90.
 //
 // A value that is not finite reaches its own stencil and no other cells (guarded loop, by taps:
 // weights inside the stencil flush to zero where the grid's axes differ much).
