@@ -472,7 +472,7 @@ int grad_cg(const gbn_plan *p) {
 // 16 x 16 ones, but halve the samples that share a window and a block's warps.  Which one gains was
 // measured on 561 plans (32^2 to 512^2, 1 to 20 frames, radial, spiral and random samples), as the
 // time with 8 x 16 bins over that with 16 x 16, geometric means: 8 coils a block 12 taps 0.94, 14
-// 0.97, 16 0.77, 4 to 10 taps 1.08, but 0.93 from 56 samples per 8 x 16 cells; 4 coils a block 8
+// 0.97, 16 0.77, 4 to 10 taps 1.08, but 0.95 from 48 samples per 8 x 16 cells; 4 coils a block 8
 // to 12 taps 0.90, 4 and 6 1.09, 14 and 16 1.22; 2 coils 1.04, 1 coil 1.10; any of them with few
 // bins (up to 224 of 16 x 16), which leave the GPU idle, 0.96.  12 coils, 64 frames of 192^2, 10
 // taps: 792 -> 587 us; 2 coils, 20 frames of 256^2, 12 taps: 89 against 144 us.  Over all of them
@@ -486,7 +486,7 @@ void interp_bins2d(gbn_plan *p) {
     bool half;
     if (W > 16) half = W <= kWideMaxW;
     else if (items <= 224) half = true;
-    else if (cg >= 8) half = W >= 12 || 128.0 * (double)p->M >= 56.0 * p->nf[0] * p->nf[1] * p->desc.n_traj;
+    else if (cg >= 8) half = W >= 12 || 128.0 * (double)p->M >= 48.0 * p->nf[0] * p->nf[1] * p->desc.n_traj;
     else half = cg >= 4 && W >= 8 && W <= 12;
     const int tile[3] = {half ? 8 : 16, 16, 1};
     make_geom(p, tile, p->gi);

@@ -32,7 +32,7 @@ def test_bins_and_interp(W, nc, nt, dense, bins):
     rng = np.random.default_rng(W + nc)
     shape = (40, 37)
     nsp, nf, tau = O.grid_params(2, *shape, eps=EPS[W])
-    M = int(np.ceil((57 if dense else 10) * nf[0] * nf[1] / 128)) * nt
+    M = int(np.ceil((49 if dense else 10) * nf[0] * nf[1] / 128)) * nt
     p = NufftPlan(2, shape, n_coil=nc, n_traj=nt, eps=EPS[W])
     for m in (M, 300, M):  # the bins follow the samples; buffers are re-used
         off = [m * g // nt for g in range(nt + 1)]
