@@ -54,6 +54,25 @@ __device__ __forceinline__ float ex2_approx(float x) {
     return y;
 }
 
+// a stencil's first cell relative to its tile (signed, periodic)
+__device__ __forceinline__ int first_plane(int c0, int o, int nf, int W) {
+    int r = c0 - o;
+    r += r < 0 ? nf : 0;
+    r -= r > nf - W ? nf : 0;
+    return r;
+}
+// Whether a weight inside the stencil, or a product of one weight an axis, can be zero in FP32:
+// ex2_approx flushes below 2^-126, products vanish below 2^-149.
+inline bool weights_flush(const Geom &g) {
+    float sum = 0.f, most = 0.f;
+    for (int d = 0; d < g.dim; ++d) {
+        const float e = g.beta2[d] * (float)(g.ns * g.ns);  // the farthest tap's exponent
+        sum += e;
+        most = e > most ? e : most;
+    }
+    return most > 125.f || sum > 147.f;
+}
+
 // --------------------------------------------------------------------------------- interp
 template <int WT, int CG>
 __global__ void __launch_bounds__(512) k_interp2d(InterpArgs a) {

@@ -6,7 +6,7 @@
 //
 // As k_interp3d_one: a warp per sample, 16 lanes read a row's taps two cells (16 bytes) at a
 // time from the even cell at or below the first, two rows a step; a cell outside the stencil
-// is left out by a select on its tap, so that a value that is not finite there does not reach the
+// is left out by a select, so that a value that is not finite there does not reach the
 // sum (and one inside does, also where the weight has flushed to zero).
 #pragma once
 
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(256) k_interp2d_wide(InterpArgs a, int vec, in
         for (int t = 0; t < 2; ++t) {
             const float d = p.y + (float)(ns - 1 - ky - t);
             const float ex = ex2_approx(-g.beta2[1] * d * d);
-            wy[t] = live && (unsigned)(ky + t) < (unsigned)W ? ex : 0.f;
+            wy[t] = live && (unsigned)(ky + t) < (unsigned)W ? ex : -1.f;  // -1: not a tap
         }
         const float4 *base = smem_iw + (rel[0] + xo) * R + (yr >> 1) + (live ? py : 0);
         float2 a0 = make_float2(0.f, 0.f), a1 = make_float2(0.f, 0.f);
@@ -87,8 +87,8 @@ __global__ void __launch_bounds__(256) k_interp2d_wide(InterpArgs a, int vec, in
             a1 = __ffma2_rn(w2, make_float2(u.z, u.w), a1);
         }
         float x = 0.f, y = 0.f;
-        if (live && (unsigned)ky < (unsigned)W) { x = wy[0] * a0.x; y = wy[0] * a0.y; }
-        if (live && (unsigned)(ky + 1) < (unsigned)W) { x = fmaf(wy[1], a1.x, x); y = fmaf(wy[1], a1.y, y); }
+        if (wy[0] >= 0.f) { x = wy[0] * a0.x; y = wy[0] * a0.y; }
+        if (wy[1] >= 0.f) { x = fmaf(wy[1], a1.x, x); y = fmaf(wy[1], a1.y, y); }
 #pragma unroll
         for (int m = 16; m > 0; m >>= 1) {
             x += __shfl_xor_sync(0xffffffffu, x, m);

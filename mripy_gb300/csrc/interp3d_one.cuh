@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(256) k_interp3d_one(InterpArgs a, int vec) {
         for (int t = 0; t < 2; ++t) {
             const float d = p.z + (float)(ns - 1 - kz - t);
             const float ex = ex2_approx(-g.beta2[2] * d * d);
-            wz[t] = live && (unsigned)(kz + t) < (unsigned)W ? ex : 0.f;
+            wz[t] = live && (unsigned)(kz + t) < (unsigned)W ? ex : -1.f;  // -1: not a tap
         }
         float wy[STEPS];
 #pragma unroll
@@ -174,10 +174,10 @@ __global__ void __launch_bounds__(256) k_interp3d_one(InterpArgs a, int vec) {
                 plane_sum(base + (size_t)kx * WY * R, __shfl_sync(0xffffffffu, myw, kx));
         }
         // a grid value that is not finite must reach the sum from inside the stencil (also where
-        // the weight has flushed to zero) and not from outside: select by tap
+        // the weight has flushed to zero) and not from outside: select
         float x = 0.f, y = 0.f;
-        if (live && (unsigned)kz < (unsigned)W) { x = wz[0] * a0.x; y = wz[0] * a0.y; }
-        if (live && (unsigned)(kz + 1) < (unsigned)W) { x = fmaf(wz[1], a1.x, x); y = fmaf(wz[1], a1.y, y); }
+        if (wz[0] >= 0.f) { x = wz[0] * a0.x; y = wz[0] * a0.y; }
+        if (wz[1] >= 0.f) { x = fmaf(wz[1], a1.x, x); y = fmaf(wz[1], a1.y, y); }
 #pragma unroll
         for (int m = 16; m > 0; m >>= 1) {
             x += __shfl_xor_sync(0xffffffffu, x, m);

@@ -183,7 +183,8 @@ cudaError_t launch_spread(const SpreadArgs &a, int64_t n_sub, int coil_group, in
     if (spread_wide_applies(a.g)) {
         for (int c0 = 0; c0 < a.g.n_coil && err == cudaSuccess; c0 += kMaxGridY) {
             const dim3 blocks((unsigned)n_sub, (unsigned)std::min(a.g.n_coil - c0, kMaxGridY));
-            k_spread2d_wide<<<blocks, kWideWarps * 32, kWideSmem, s>>>(a, c0);
+            if (weights_flush(a.g)) k_spread2d_wide<true><<<blocks, kWideWarps * 32, kWideSmem, s>>>(a, c0);
+            else k_spread2d_wide<false><<<blocks, kWideWarps * 32, kWideSmem, s>>>(a, c0);
             err = cudaGetLastError();
         }
         return err;
@@ -191,10 +192,17 @@ cudaError_t launch_spread(const SpreadArgs &a, int64_t n_sub, int coil_group, in
     // few-coil 3-D kernel
     if (few_applies(a.g)) {
         const int nc = a.g.n_coil;
+        if (weights_flush(a.g)) {
+            auto kern = nc == 1   ? (a.real ? k_spread3d_few<0, 1, true, true> : k_spread3d_few<0, 1, false, true>)
+                        : nc == 2 ? k_spread3d_few<0, 2, false, true>
+                                  : k_spread3d_few<0, 3, false, true>;
+            kern<<<(unsigned)n_sub, kFewWarps * 32, few_smem_bytes(nc), s>>>(a);
+            return cudaGetLastError();
+        }
         GBN_DISPATCH_W(a.g.W, {
-            auto kern = nc == 1   ? (a.real ? k_spread3d_few<WT, 1, true> : k_spread3d_few<WT, 1, false>)
-                        : nc == 2 ? k_spread3d_few<WT, 2, false>
-                                  : k_spread3d_few<WT, 3, false>;
+            auto kern = nc == 1   ? (a.real ? k_spread3d_few<WT, 1, true, false> : k_spread3d_few<WT, 1, false, false>)
+                        : nc == 2 ? k_spread3d_few<WT, 2, false, false>
+                                  : k_spread3d_few<WT, 3, false, false>;
             kern<<<(unsigned)n_sub, kFewWarps * 32, few_smem_bytes(nc), s>>>(a);
             err = cudaGetLastError();
         });

@@ -18,8 +18,8 @@
 // a 1024^2 grid 210 -> 100; 3 coils, 20 frames of 256^2, 14,800 each 416 -> 164; only sparse random
 // samples (15 a tile, 2 coils, 20 frames of 512^2) 79 -> 90.
 //
-// A value that is not finite reaches its own stencil and no other cells (guarded loop, by taps:
-// weights inside the stencil flush to zero where the grid's axes differ much).
+// A value that is not finite reaches its own stencil and no other cells (guarded loop; by the
+// taps in an instance of its own, as k_spread3d_few).
 #pragma once
 
 #include "grid2d_kernels.cuh"
@@ -30,6 +30,7 @@ constexpr int kWideTile = 32, kWideWarps = 4, kWideStride = 68;  // floats per s
 constexpr size_t kWideSmem = (size_t)kWideWarps * 32 * kWideStride * sizeof(float);
 static_assert(kWideSmem >= 2 * 32 * 33 * sizeof(float2), "two partial tiles");
 
+template <bool TAPS>
 __global__ void __launch_bounds__(kWideWarps * 32, 4) k_spread2d_wide(SpreadArgs a, int coil0) {
     extern __shared__ float4 smem_wide[];
     const Geom &g = a.g;
@@ -97,18 +98,36 @@ __global__ void __launch_bounds__(kWideWarps * 32, 4) k_spread2d_wide(SpreadArgs
         const unsigned bad = __ballot_sync(0xffffffffu, !(isfinite(v.x) && isfinite(v.y)));
         __syncwarp();
         if (base + kWideWarps * 32 < sub.z) fetch(base + kWideWarps * 32, p, v);
-        if (bad) {  // guarded: only the cells inside the stencil
+        if (TAPS && bad) {
+            int r2[2];
+            unpack_cells(2, __float_as_uint(a.pts[(int64_t)sub.y + min(base + lane, sub.z - 1)].w), c0[0], c0[1], c0[2]);
+#pragma unroll
+            for (int d = 0; d < 2; ++d) r2[d] = first_plane(c0[d], o[d], g.nf[d], W);
 #pragma unroll 1
             for (int s = 0; s < n; ++s) {
                 const float *w = st + s * kWideStride;
                 const float wx = w[lane], vx = w[64], vy = w[65];
-                const int sx = __shfl_sync(0xffffffffu, r[0], s), sy = __shfl_sync(0xffffffffu, r[1], s);
+                const int sx = __shfl_sync(0xffffffffu, r2[0], s), sy = __shfl_sync(0xffffffffu, r2[1], s);
                 if ((unsigned)(lane - sx) >= (unsigned)W) continue;
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     const float ga = wx * w[32 + 2 * i], gb = wx * w[33 + 2 * i];
                     if ((unsigned)(2 * i - sy) < (unsigned)W) { re[i].x = fmaf(ga, vx, re[i].x); im[i].x = fmaf(ga, vy, im[i].x); }
                     if ((unsigned)(2 * i + 1 - sy) < (unsigned)W) { re[i].y = fmaf(gb, vx, re[i].y); im[i].y = fmaf(gb, vy, im[i].y); }
+                }
+            }
+            continue;
+        }
+        if (bad) {  // guarded: only the cells inside the stencil
+#pragma unroll 1
+            for (int s = 0; s < n; ++s) {
+                const float *w = st + s * kWideStride;
+                const float wx = w[lane], vx = w[64], vy = w[65];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const float ga = wx * w[32 + 2 * i], gb = wx * w[33 + 2 * i];
+                    if (ga != 0.f) { re[i].x = fmaf(ga, vx, re[i].x); im[i].x = fmaf(ga, vy, im[i].x); }
+                    if (gb != 0.f) { re[i].y = fmaf(gb, vx, re[i].y); im[i].y = fmaf(gb, vy, im[i].y); }
                 }
             }
             continue;

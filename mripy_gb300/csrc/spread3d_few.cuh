@@ -1,5 +1,5 @@
 // 3-D spread (type-1 gridding) of 1 to 3 coils with the output tile in registers:
-// k_spread3d_few<WT, NC, REAL>.
+// k_spread3d_few<WT, NC, REAL, TAPS>.
 //
 // What bounds it: FP32 issue.  A sample's W^3 taps are 4 W^3 flops a coil against 16 + 8 NC
 // bytes of input, so the cells have to stay out of shared memory: read-modify-write of a
@@ -21,8 +21,10 @@
 // REAL: the samples' imaginary parts are zero (density compensation): half the FMAs.
 //
 // A value that is not finite reaches the cells of its own stencil and no others, as with the
-// kernels that walk the stencil: a batch with such a sample takes the guarded loop, which goes by
-// the taps (weights inside the stencil flush to zero where a grid's axes differ much).
+// kernels that walk the stencil: a batch with such a sample takes the guarded loop, which skips
+// the zero weights instead of multiplying by them.  TAPS: the loop goes by the taps instead, for
+// grids whose axes differ so much that weights inside the stencil are zero in FP32 (an instance of
+// its own: with the comparisons of taps the others take up to 2.6 % longer, by their registers).
 #pragma once
 
 #include "grid2d_kernels.cuh"
@@ -50,7 +52,7 @@ constexpr size_t few_smem_bytes(int nc) {
 __host__ __device__ constexpr int few_blocks(int nc, bool real) { return real ? 6 : (nc <= 2 ? 4 : 3); }
 
 // The lane's sample staged: first taps relative to the tile (signed), then the tile-plane
-// weights.  Returns the first taps, 8 bits each, offset by 16 (few_tap).
+// weights.  Returns r[2] (z) for the half masks.
 template <int WT, int TZ>
 __device__ __forceinline__ int few_stage(const Geom &g, const int o[3], const float4 &p, float4 *mine) {
     const int W = WT ? WT : g.W, ns = g.ns;
@@ -78,9 +80,8 @@ __device__ __forceinline__ int few_stage(const Geom &g, const int o[3], const fl
         }
         mine[q] = make_float4(w4[0], w4[1], w4[2], w4[3]);
     }
-    return (r[0] + 16) | (r[1] + 16) << 8 | (r[2] + 16) << 16;
+    return r[2];
 }
-__device__ __forceinline__ int few_tap(int packed, int d) { return (packed >> 8 * d & 255) - 16; }
 
 __device__ __forceinline__ void few_load_z(const float *w, float2 (&wz)[4]) {
     const float4 a = *reinterpret_cast<const float4 *>(w), b = *reinterpret_cast<const float4 *>(w + 4);
@@ -91,7 +92,7 @@ __device__ __forceinline__ void few_load_z(const float *w, float2 (&wz)[4]) {
 }
 
 // --------------------------------------------------------------------------------- spread
-template <int WT, int NC, bool REAL>
+template <int WT, int NC, bool REAL, bool TAPS>
 __global__ void __launch_bounds__(kFewWarps * 32, few_blocks(NC, REAL)) k_spread3d_few(SpreadArgs a) {
     constexpr int TZ = few_tz(NC), ZP = TZ / 2, ST = few_stride(NC), CELLS = few_cells(NC), RI = REAL ? 1 : 2;
     extern __shared__ float4 smem_few[];
@@ -141,8 +142,7 @@ __global__ void __launch_bounds__(kFewWarps * 32, few_blocks(NC, REAL)) k_spread
     for (int base = warp * 32; base < sub.z; base += kFewWarps * 32) {
         const int n = min(32, sub.z - base);
         __syncwarp();  // the previous batch is consumed
-        const int taps = few_stage<WT, TZ>(g, o, p, reinterpret_cast<float4 *>(st + lane * ST));
-        const int rz = few_tap(taps, 2);
+        const int rz = few_stage<WT, TZ>(g, o, p, reinterpret_cast<float4 *>(st + lane * ST));
         bool fin = true;
 #pragma unroll
         for (int c = 0; c < NC; ++c)
@@ -158,13 +158,17 @@ __global__ void __launch_bounds__(kFewWarps * 32, few_blocks(NC, REAL)) k_spread
         __syncwarp();
         if (base + kFewWarps * 32 < sub.z) fetch(base + kFewWarps * 32, p, v);
 
-        if (bad) {  // guarded: only the cells inside the stencil
+        if (TAPS && bad) {
+            int c0[3], r3[3];
+            unpack_cells(3, __float_as_uint(a.pts[(int64_t)sub.y + min(base + lane, sub.z - 1)].w), c0[0], c0[1], c0[2]);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) r3[d] = first_plane(c0[d], o[d], g.nf[d], W);
 #pragma unroll 1
             for (int s = 0; s < n; ++s) {
                 const float *w = st + s * ST;
                 const float t[2] = {w[lx] * w[8 + 2 * yq], w[lx] * w[9 + 2 * yq]};
-                const int ts = __shfl_sync(0xffffffffu, taps, s);
-                const int sx = few_tap(ts, 0), sy = few_tap(ts, 1), sz = few_tap(ts, 2);
+                const int sx = __shfl_sync(0xffffffffu, r3[0], s), sy = __shfl_sync(0xffffffffu, r3[1], s);
+                const int sz = __shfl_sync(0xffffffffu, r3[2], s);
 #pragma unroll
                 for (int c = 0; c < NC; ++c)
 #pragma unroll
@@ -181,6 +185,29 @@ __global__ void __launch_bounds__(kFewWarps * 32, few_blocks(NC, REAL)) k_spread
                                     m.y = fmaf(t[r] * w[17 + 2 * z], u, m.y);
                             }
                         }
+                    }
+            }
+            continue;
+        }
+        if (bad) {  // guarded: only the cells inside the stencil
+#pragma unroll 1
+            for (int s = 0; s < n; ++s) {
+                const float *w = st + s * ST;
+                const float t[2] = {w[lx] * w[8 + 2 * yq], w[lx] * w[9 + 2 * yq]};
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+#pragma unroll
+                    for (int k = 0; k < RI; ++k) {
+                        const float u = w[16 + TZ + RI * c + k];
+#pragma unroll
+                        for (int r = 0; r < 2; ++r)
+#pragma unroll
+                            for (int z = 0; z < ZP; ++z) {
+                                const float ga = t[r] * w[16 + 2 * z], gb = t[r] * w[17 + 2 * z];
+                                float2 &m = acc[c][k][r][z];
+                                if (ga != 0.f) m.x = fmaf(ga, u, m.x);
+                                if (gb != 0.f) m.y = fmaf(gb, u, m.y);
+                            }
                     }
             }
             continue;
