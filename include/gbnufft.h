@@ -69,13 +69,15 @@ typedef struct {
     int32_t n_traj;         /* trajectory groups (frames/slices), ragged sample counts */
     /* tuning (0 = library default; the autotuner fills these) */
     int32_t spread_tile[3]; /* output tile of the spread kernel, cells per dim */
-    int32_t interp_tile[3]; /* home bin of the interp kernel, cells per dim */
+    int32_t interp_tile[3]; /* home bin of the interp kernel, cells per dim (0 in 2-D: chosen by
+                               gbn_set_points from taps, coils and samples) */
     int32_t max_subproblem; /* samples per thread block before a bin is split */
     int32_t coil_group;     /* coils per spread thread block: 1, 2, 4 or 8 */
     int32_t threads;        /* threads per spread block: 128, 256 or 512 */
     int32_t interp_threads; /* threads per interp block: 128, 256 or 512 */
     int32_t interp_coil_group; /* coils per interp thread block: 1, 2, 4 or 8 (0: the
-                                  group that pads the coil count least) */
+                                  group that pads the coil count least; in 3-D one coil
+                                  where taps, coils, samples and bins make that faster) */
     int32_t interp_staging;    /* 2-D interp windows and 3-D interp planes: 0 = tensor-
                                   memory-access copies where the grid allows (default),
                                   1 = thread loads */
