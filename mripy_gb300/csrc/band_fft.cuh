@@ -2,12 +2,12 @@
 // k_fft_rows_in (image -> transformed grid rows), k_fft_cols (a strided axis, in place) and
 // k_fft_rows_out / k_fft_rows_sense (grid rows -> image).
 //
-// What bounds them: the bytes moved, through L1 and HBM.  An oversampled grid is zero outside the image band before the
-// forward transform, and only the band is read after the inverse one.  A pad kernel, a
-// library transform over the whole grid and a crop kernel move the grid 5 (2-D) to 7 (3-D)
-// times; here an axis is transformed only on the band of the axes that come later, so type 2
-// reads the image once and moves 1/2 + 1/2 + 1 grids in 2-D (1/4 + 1/4 + 1/2 + 1/2 + 1 in
-// 3-D), and type 1 the same backwards.
+// What bounds them: the bytes moved, through L1 and HBM.  An oversampled grid is zero outside the
+// image band before the forward transform, and only the band is read after the inverse one.  A
+// pad kernel, a library transform over the whole grid and a crop kernel move the grid 5 (2-D) to
+// 7 (3-D) times; here an axis is transformed only on the band of the axes that come later, so
+// type 2 reads the image once and moves 1/2 + 1/2 + 1 grids in 2-D (1/4 + 1/4 + 1/2 + 1/2 + 1
+// in 3-D), and type 1 the same backwards.
 //
 // A line of N = R1 R2 cells is two register passes with one exchange through shared memory:
 // a thread reads the R1 cells j + r R2 straight from the image or grid, transforms them,
@@ -28,7 +28,8 @@
 // 192^2 in 1.14 -> 0.49 ms and out 1.02 -> 0.48 ms; 8 images of 128^3 in 0.96 -> 0.56 ms, out
 // 0.82 -> 0.55 ms.  The strided passes run at 69 to 77 % of the copy bandwidth with the L1/shared
 // pipe at 73 to 78 %, two to four blocks per SM whose load, transform and store phases overlap
-// only across blocks; the row passes at 3.3 TB/s wait for loads and barriers.  Error against 64 bits: 1.3e-7 to 1.7e-7 (cuFFT 2.0e-7 to 2.6e-7).
+// only across blocks; the row passes at 3.3 TB/s wait for loads and barriers.  Error against 64
+// bits: 1.3e-7 to 1.7e-7 (cuFFT 2.0e-7 to 2.6e-7).
 //
 // The inverse transform is the forward one with real and imaginary parts swapped on the way
 // in and out.
