@@ -404,27 +404,39 @@ int run_spread(gbn_plan *p, const void *c, gbn_layout L, const float *weight, fl
 }
 
 // 3-D interps off the tensor cores: whether a block per coil (interp3d_one.cuh) is faster than
-// groups of 2 (k_interp3d), 4 or 8 coils (the plane-streaming kernel).  It is from 8 taps up to 3
-// coils; for 4 to 6 coils with few work items, which leave the GPU idle in groups, in grids of
-// at most 4096 bins, or with many samples a bin: below that a bin's samples read their taps from
-// the grid itself, which in large grids no longer come from L1 (10 taps, whose lanes are all
-// used, are the faster all the same).  Few taps leave most of its lanes idle.  Measured on 470
-// plans (1 to 7 coils, 40^3 to 192^3 grids, 1 to 250 samples a bin, radial and random), groups ->
-// a block per coil: 4 taps, 6 coils, 361,000 samples on 128^3 365 -> 810 us, 2,400 on 40^3 25 -> 17;
-// 6 taps, 4 coils, 108,000 on 128^3 165 -> 205, 2,800 on 96^3 41 -> 25; 8 taps, 4 coils, 131,000
-// on 192^3 392 -> 706, 7,800 radial in three 96^3 76 -> 40; 10 taps, 4 coils, 192,000 on 128^3 487
-// -> 384; 12 taps, 4 coils, 29,500 on 192^3 385 -> 601, 9,500 radial 120 -> 89; 14 taps, 6 coils,
-// 201,000 on 192^3 1880 -> 3747, 436,000 radial on 128^3 3356 -> 3109.
+// groups of 2 (k_interp3d), 4 or 8 coils (the plane-streaming kernel).  It is the faster with 8
+// and more taps where a bin's samples share a window, and where few work items leave the GPU idle in
+// groups; a bin of few samples reads its taps from the grid itself, which is slower as soon as the
+// coils' grids no longer come from the L2 cache (T bins are 4096 T cells of a coil; 10 taps, whose
+// lanes are all used, are the faster all the same).  Few taps leave most of its lanes idle.
+// Measured on 470 plans of 1 to 7 coils and 580 of 2 to 6 (40^3 to 256^3 grids, 0.1 to 3000 samples
+// a bin, radial, spiral and random), groups -> a block per coil: 4 taps, 6 coils, 361,000 samples on
+// 128^3 365 -> 810 us, 2,400 on 40^3 25 -> 17; 6 taps, 2 coils, 138,000 in four 128^3 376 -> 226, 3
+// coils, 124,000 on 80^3 168 -> 119, 4 coils, 108,000 on 128^3 165 -> 205; 8 taps, 3 coils, 15,400
+// random on 172^3 179 -> 277, 4 coils, 131,000 on 192^3 392 -> 706, 7,800 radial in three 96^3 76 ->
+// 40, 5 coils, 172,000 radial on 144^3 509 -> 415; 10 taps, 4 coils, 192,000 on 128^3 487 -> 384; 12
+// taps, 4 coils, 29,500 on 192^3 385 -> 601, 9,500 radial 120 -> 89, 6 coils, 452,000 random in two
+// 192^3 2417 -> 3534; 14 taps, 3 coils, 19,000 random on 192^3 468 -> 898, 692,000 spiral 3102 -> 2826,
+// 6 coils, 201,000 on 192^3 1880 -> 3747.  Over the 580 the choice takes 1.01 times the faster one's time.
 bool interp_one_coil(const gbn_plan *p) {
     if (p->dim != 3 || !interp3d_one_applies(p->gi)) return false;
     const int W = p->gi.W;
     const int64_t n = p->desc.n_coil, M = p->M, T = (int64_t)p->gi.ntiles * p->gi.n_traj;
     const int64_t items = p->points_set ? p->n_interp_sub : std::min(T, M);  // (at most, while binning)
     if (W <= 4) return n * M <= 32768 || (n <= 2 && M <= 8 * T);
-    if (W <= 6) return n == 1 || n * M <= 262144;
-    if (n <= 3 || W == 10) return true;
-    if (W == 8) return T <= 4096 || items <= 1700;
-    if (W == 12) return n == 5 || T <= 4096 || items <= 2100 || M >= 8 * T;
+    if (W <= 6) {
+        if (n == 2) return M <= 128 * T;
+        if (n == 3) return T <= 12000 || items <= 12000 || M >= 32 * T;
+        return n == 1 || n * M <= 262144 || (n == 5 && T <= 4096);
+    }
+    if (n <= 2 || W == 10) return true;
+    if (n == 3) {
+        if (W == 8) return T <= 8192 || items <= 2200 || M >= 32 * T;
+        if (W == 12) return T <= 16384 || items <= 4000 || M >= 16 * T;
+        return T < 4096 || items <= (T <= 8000 ? 3800 : 2200) || M >= 32 * T;
+    }
+    if (W == 8) return T <= 4096 || items <= 1700 || (T <= 8000 && M >= 20 * T);
+    if (W == 12) return n == 5 || T <= 4096 || items <= 2100 || M >= (T <= 8000 ? 8 : 24) * T;
     return T < 4096 || items <= 1200 || (n >= 5 && M >= 64 * T);
 }
 
