@@ -83,6 +83,7 @@ struct gbn_plan {
     Geom gs{}, gi{};
     int coil_group = 1, threads = 256, interp_threads = 256, max_sub = 256, interp_coil_group = 0;
     int interp_max_sub = 1 << 30;  // interp work items where the spread's own size is longer
+    int interp_items = 256;  // most samples of an interp work item (set_points)
     bool auto_bins = false;  // 2-D: set_points chooses the interp bins (interp_bins2d)
     int interp_staging = 0;  // 0: tensor copies where the grid allows, 1: thread loads
     int interp_variant = 0;  // 3-D, 8 coils: 0 library choice, 1 interp bins, 2 tensor cores
@@ -407,8 +408,8 @@ int run_spread(gbn_plan *p, const void *c, gbn_layout L, const float *weight, fl
 // groups of 2 (k_interp3d), 4 or 8 coils (the plane-streaming kernel).  It is the faster with 8
 // and more taps where a bin's samples share a window, and where few work items leave the GPU idle in
 // groups; a bin of few samples reads its taps from the grid itself, which is slower as soon as the
-// coils' grids no longer come from the L2 cache (T bins are 4096 T cells of a coil; 10 taps, whose
-// lanes are all used, are the faster all the same).  Few taps leave most of its lanes idle.
+// coils' grids no longer come from the L2 cache (a bin is 4 KB of a coil; 10 taps, whose lanes are
+// all used, are the faster all the same).  Few taps leave most of its lanes idle.
 // Measured on 470 plans of 1 to 7 coils and 580 of 2 to 6 (40^3 to 256^3 grids, 0.1 to 3000 samples
 // a bin, radial, spiral and random), groups -> a block per coil: 4 taps, 6 coils, 361,000 samples on
 // 128^3 365 -> 810 us, 2,400 on 40^3 25 -> 17; 6 taps, 2 coils, 138,000 in four 128^3 376 -> 226, 3
@@ -732,6 +733,7 @@ int set_points_impl(gbn_plan *p, int dtype, const void *x, const void *y, const 
     const int interp_max_sub = interp3d_planes_smem(p->gi, interp_cg(p), p->interp_threads) > 0
                                    ? std::min(p->max_sub, kPlaneSamples)
                                    : std::min(p->max_sub, p->interp_max_sub);
+    p->interp_items = interp_max_sub;
     p->spread_items_interleaved = spread_interleaved(p);
     SubsJob js{}, ji{};
     js.count = scount;
@@ -1449,6 +1451,10 @@ int gbn_interp_grad_coords(gbn_plan *p, const void *grid, const void *grad_c, gb
     if (p->auto_bins && p->desc.interp_threads <= 0 && p->gi.tile[0] < std::min(16, p->nf[0]) &&
         p->n_interp_sub * ((p->desc.n_coil + cg - 1) / cg) >= 1024)
         threads = 256;
+    // 3-D, a thread a sample: as many of a bin's items as give each thread one (the plane-streaming
+    // interp's have 64).  6 taps, 4 coils, 1.7 M samples in four 64^3 grids 1471 us, item by item 3031; 6
+    // coils, 138,000 on 96^3 313 and 448.
+    if (p->dim == 3) a.span = (unsigned)std::max(1, std::min(threads, 256) / p->interp_items);
     GBN_CUDA(launch_interp_grad(a, p->n_interp_sub, cg, threads, s));
     return GBN_OK;
 }

@@ -190,6 +190,7 @@ struct GradArgs {
     int64_t c_elem, c_coil;
     float *out;               // (M, dim)
     float scale;              // df
+    unsigned span = 1;        // 1-D, 3-D and above 16 taps: items of a bin that one block takes
 };
 // the 3-D tensor-core interp: the spread's tiles and (sample, tile) work lists
 struct MmaInterpArgs {

@@ -296,6 +296,16 @@ __global__ void __launch_bounds__(256) k_interp_grad(GradArgs a, float dsc0, flo
     extern __shared__ float2 win[];
     const Geom &g = a.g;
     const int4 sub = a.subs[blockIdx.x];
+    // up to a.span items of a bin, which follow each other in the list, are one block's
+    int count = sub.z;
+    if (a.span > 1) {
+        if (!(sub.w & kFirstFlag) && blockIdx.x % a.span) return;
+        for (unsigned b = blockIdx.x + 1; b % a.span && b < gridDim.x; ++b) {
+            const int4 next = a.subs[b];
+            if (next.w & kFirstFlag) break;
+            count += next.z;
+        }
+    }
     const int cg0 = blockIdx.y * CG;
     const int grp = sub.x / g.ntiles;
     int o[3], e[3], wd[3];
@@ -308,9 +318,9 @@ __global__ void __launch_bounds__(256) k_interp_grad(GradArgs a, float dsc0, flo
     constexpr int WA = WT ? WT : kMaxW;
     int lanes = 1;  // a sample's lanes, which share its rows of taps
     if (WT == 0)
-        while (lanes < 16 && 2 * lanes * sub.z <= (int)blockDim.x) lanes *= 2;
+        while (lanes < 16 && 2 * lanes * count <= (int)blockDim.x) lanes *= 2;
     const int part = threadIdx.x & (lanes - 1);
-    for (int i = threadIdx.x / lanes; i < sub.z; i += blockDim.x / lanes) {
+    for (int i = threadIdx.x / lanes; i < count; i += blockDim.x / lanes) {
         const int64_t li = (int64_t)sub.y + i;
         const float4 p = a.pts[li];
         const uint32_t j = a.idx[li];
