@@ -47,9 +47,11 @@ namespace {
 #define GBN_CUDA(call)                                                                          \
     do {                                                                                        \
         cudaError_t e_ = (call);                                                                \
-        if (e_ != cudaSuccess)                                                                  \
-            return fail(e_ == cudaErrorMemoryAllocation ? GBN_ERR_ALLOC : GBN_ERR_CUDA,          \
-                        std::string(#call) + ": " + cudaGetErrorString(e_));                     \
+        if (e_ != cudaSuccess) {                                                                \
+            cudaGetLastError(); /* or the next launch of any plan would report it */            \
+            return fail(e_ == cudaErrorMemoryAllocation ? GBN_ERR_ALLOC : GBN_ERR_CUDA,         \
+                        std::string(#call) + ": " + cudaGetErrorString(e_));                    \
+        }                                                                                       \
     } while (0)
 
 #define GBN_FFT(call)                                                                           \
